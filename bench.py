@@ -169,7 +169,8 @@ class ClockSampler:
 # framebuffer read-modify-write per pixel.
 BYTES_PER_WORK = {"nodes": 64, "tris": 48, "rays": 72, "point_cand": 16, "point_hit": 128, "beam_cand": 48,
                   "beam_hit": 128, "vertex_loads": 128}
-# The PB2D, BB1D and BP2D searches walk the maps' 32-byte compressed nodes.
+# The PB2D, BB1D and BP2D searches count 32 bytes a node test (they read the
+# maps' 48-byte four-wide nodes, shared by the queries of a group).
 COMPRESSED_NODE_KERNELS = ("pb2d_query", "bb1d_query", "bp2d_query")
 
 

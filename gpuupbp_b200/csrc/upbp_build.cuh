@@ -255,38 +255,62 @@ UPBP_D unsigned qnode_quantize(float v, float origin, float step, bool upper)
     return (unsigned)q;
 }
 
-// Compressed copy of the n - 1 internal nodes of a tree built with
-// one-primitive leaves (every child link is gamma or gamma + 1).
-__global__ void k_quantize(const BvhNode* nodes, int n_internal, QNode* q)
+// Four-wide compressed nodes of the n - 1 internal nodes of a tree built with
+// one-primitive leaves (every child link is gamma or gamma + 1): node i
+// holds the boxes of the children of its own children.  Every node gets one,
+// although a walk from the root reaches every other level only: picking
+// them would take a pass over the tree per level.
+__global__ void k_quantize(const BvhNode* nodes, int n_internal, QNode4* q)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_internal) return;
-    const float4 a = nodes[i].a, b = nodes[i].b, c = nodes[i].c;
-    const int4 k = nodes[i].link;
-    const float lo[2][3] = {{a.x, a.y, a.z}, {b.z, b.w, c.x}};
-    const float hi[2][3] = {{a.w, b.x, b.y}, {c.y, c.z, c.w}};
-    float org[3], step[3];
+    float lo[4][3], hi[4][3];
+    unsigned link[2];
+    auto boxes = [&](const BvhNode& n, int c) {
+        const float4 a = n.a, b = n.b, d = n.c;
+        const float l[2][3] = {{a.x, a.y, a.z}, {b.z, b.w, d.x}}, h[2][3] = {{a.w, b.x, b.y}, {d.y, d.z, d.w}};
+        for (int s = 0; s < 2; s++)
+            for (int ax = 0; ax < 3; ax++) {
+                lo[c + s][ax] = l[s][ax];
+                hi[c + s][ax] = h[s][ax];
+            }
+    };
+    boxes(nodes[i], 0);
+    const float lo1[3] = {lo[1][0], lo[1][1], lo[1][2]}, hi1[3] = {hi[1][0], hi[1][1], hi[1][2]};
+    float org[3], top[3], step[3];
     unsigned ebits = 0;
     for (int ax = 0; ax < 3; ax++) {
-        org[ax] = fminf(lo[0][ax], lo[1][ax]);
-        const unsigned e = qnode_exponent(org[ax], fmaxf(hi[0][ax], hi[1][ax]));
+        org[ax] = fminf(lo[0][ax], lo1[ax]);
+        top[ax] = fmaxf(hi[0][ax], hi1[ax]);
+        const unsigned e = qnode_exponent(org[ax], top[ax]);
         step[ax] = qnode_step(e);
         ebits |= e << (8 * ax);
     }
-    unsigned bytes[12];
-    for (int ch = 0; ch < 2; ch++)
-        for (int ax = 0; ax < 3; ax++) {
-            bytes[6 * ch + ax] = qnode_quantize(lo[ch][ax], org[ax], step[ax], false);
-            bytes[6 * ch + 3 + ax] = qnode_quantize(hi[ch][ax], org[ax], step[ax], true);
+    const int kid[2] = {nodes[i].link.x, nodes[i].link.y};
+    for (int s = 1; s >= 0; s--) {
+        if (kid[s] < 0) {
+            link[s] = (unsigned)leaf_first(kid[s]) | kQnodeLeaf0 | kQnodeSingle;
+            for (int ax = 0; ax < 3; ax++) {  // child 0 of its pair; the other one does not count
+                lo[2 * s][ax] = lo[2 * s + 1][ax] = s ? lo1[ax] : lo[0][ax];
+                hi[2 * s][ax] = hi[2 * s + 1][ax] = s ? hi1[ax] : hi[0][ax];
+            }
+        } else {
+            const int4 k = nodes[kid[s]].link;
+            boxes(nodes[kid[s]], 2 * s);
+            link[s] = (unsigned)(k.x < 0 ? leaf_first(k.x) : k.x) | (k.x < 0 ? kQnodeLeaf0 : 0u) |
+                      (k.y < 0 ? kQnodeLeaf1 : 0u);
         }
-    uint4 w;
-    w.x = bytes[0] | bytes[1] << 8 | bytes[2] << 16 | bytes[3] << 24;
-    w.y = bytes[4] | bytes[5] << 8 | bytes[6] << 16 | bytes[7] << 24;
-    w.z = bytes[8] | bytes[9] << 8 | bytes[10] << 16 | bytes[11] << 24;
-    const unsigned g = (unsigned)(k.x < 0 ? leaf_first(k.x) : k.x);
-    w.w = g | (k.x < 0 ? 1u << 30 : 0u) | (k.y < 0 ? 1u << 31 : 0u);
+    }
+    unsigned w[6] = {0, 0, 0, 0, 0, 0};
+    for (int c = 0; c < 4; c++)
+        for (int ax = 0; ax < 3; ax++) {
+            const unsigned l = qnode_quantize(lo[c][ax], org[ax], step[ax], false);
+            const unsigned h = qnode_quantize(hi[c][ax], org[ax], step[ax], true);
+            w[2 * ax + c / 2] |= (l | h << 8) << (16 * (c & 1));
+        }
     q[i].a = make_float4(org[0], org[1], org[2], __uint_as_float(ebits));
-    q[i].b = w;
+    q[i].b = make_uint4(w[0], w[1], w[2], w[3]);
+    q[i].c = make_uint4(w[4], w[5], link[0], link[1]);
 }
 
 // Leaf-order payloads.
@@ -344,23 +368,15 @@ __global__ void k_chunk_expand(const unsigned* counts, const unsigned* offsets, 
     for (unsigned k = 0; k < c; k++) chunks[off + k] = make_uint2(b, k | (c << 16));
 }
 
-// Leaf payload of the chunked beam map: (origin, length), (direction, bits),
-// (t0, t1, medium id bits, chunk k | chunk count << 16) where bits = beam
-// index | BB1D-eligible << 31.
+// Leaf payload of the chunked beam map (BeamMap::chunk).
 __global__ void k_gather_chunks(const uint2* chunks, const BeamRec* beams, const unsigned* vals, unsigned n,
-                                unsigned bb1d_paths, float4* out)
+                                unsigned bb1d_paths, uint2* out)
 {
     const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint2 ch = chunks[vals[s]];
-    const unsigned b = ch.x;
-    const float4 q0 = beams[b].q[0], q1 = beams[b].q[1];
-    const unsigned path_idx = __float_as_uint(beams[b].q[3].z);
-    const unsigned bits = b | (path_idx < bb1d_paths ? 0x80000000u : 0u);
-    const unsigned k = ch.y & 0xffffu, c = ch.y >> 16;
-    out[3 * s] = q0;
-    out[3 * s + 1] = make_float4(q1.x, q1.y, q1.z, __uint_as_float(bits));
-    out[3 * s + 2] = make_float4(chunk_t(q0.w, k, c), chunk_t(q0.w, k + 1, c), q1.w, __uint_as_float(ch.y));
+    const unsigned path_idx = __float_as_uint(beams[ch.x].q[3].z);
+    out[s] = make_uint2(ch.x | (path_idx < bb1d_paths ? 0x80000000u : 0u), ch.y);
 }
 
 // Scratch owned by a context, sized for the largest build it will run.

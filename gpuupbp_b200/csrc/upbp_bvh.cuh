@@ -102,60 +102,6 @@ UPBP_D NodeBoxes load_node(const BvhNode* nodes, int i)
     return r;
 }
 
-// A compressed node decoded into the children's boxes (each containing the
-// exact box) and links in BvhNode form.
-UPBP_D NodeBoxes load_qnode(const QNode* q, int i)
-{
-    const float4 a = __ldg(&q[i].a);
-    const uint4 b = __ldg(&q[i].b);
-    const unsigned e = __float_as_uint(a.w);
-    const float sx = qnode_step(e & 0xffu), sy = qnode_step((e >> 8) & 0xffu), sz = qnode_step((e >> 16) & 0xffu);
-    NodeBoxes r;
-    r.llo = make_float3(qnode_plane(b.x, 0, sx, a.x), qnode_plane(b.x, 1, sy, a.y), qnode_plane(b.x, 2, sz, a.z));
-    r.lhi = make_float3(qnode_plane(b.x, 3, sx, a.x), qnode_plane(b.y, 0, sy, a.y), qnode_plane(b.y, 1, sz, a.z));
-    r.rlo = make_float3(qnode_plane(b.y, 2, sx, a.x), qnode_plane(b.y, 3, sy, a.y), qnode_plane(b.z, 0, sz, a.z));
-    r.rhi = make_float3(qnode_plane(b.z, 1, sx, a.x), qnode_plane(b.z, 2, sy, a.y), qnode_plane(b.z, 3, sz, a.z));
-    const int g = (int)(b.w & 0x3fffffffu);
-    r.l = (b.w >> 30) & 1u ? leaf_link(g, 1) : g;
-    r.r = (b.w >> 31) ? leaf_link(g + 1, 1) : g + 1;
-    return r;
-}
-
-// Segment [tmin, tmax] of a ray (inv = 1/d, oinv = o * inv) against both
-// children of compressed node i, the dequantisation folded into the plane
-// distances: a plane origin + q * step lies at t = q * (step * inv) +
-// (origin * inv - oinv), one multiply-add per plane after six per node.
-// The rounding differs from slab() on the decoded planes by a few units in
-// the last place of t, far inside the margins the stored boxes carry.
-UPBP_D void qnode_slab(const QNode* q, int i, float3 inv, float3 oinv, float tmin, float tmax, bool& hl, bool& hr,
-                       int& l, int& r)
-{
-    const float4 a = __ldg(&q[i].a);
-    const uint4 b = __ldg(&q[i].b);
-    const unsigned e = __float_as_uint(a.w);
-    const float sx = qnode_step(e & 0xffu) * inv.x, sy = qnode_step((e >> 8) & 0xffu) * inv.y,
-                sz = qnode_step((e >> 16) & 0xffu) * inv.z;
-    const float ox = fmaf(a.x, inv.x, -oinv.x), oy = fmaf(a.y, inv.y, -oinv.y), oz = fmaf(a.z, inv.z, -oinv.z);
-    auto t = [](unsigned word, int byte, float s, float o) { return fmaf((float)((word >> (8 * byte)) & 0xffu), s, o); };
-    {
-        const float x0 = t(b.x, 0, sx, ox), y0 = t(b.x, 1, sy, oy), z0 = t(b.x, 2, sz, oz);
-        const float x1 = t(b.x, 3, sx, ox), y1 = t(b.y, 0, sy, oy), z1 = t(b.y, 1, sz, oz);
-        const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-        const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax));
-        hl = tn <= tf;
-    }
-    {
-        const float x0 = t(b.y, 2, sx, ox), y0 = t(b.y, 3, sy, oy), z0 = t(b.z, 0, sz, oz);
-        const float x1 = t(b.z, 1, sx, ox), y1 = t(b.z, 2, sy, oy), z1 = t(b.z, 3, sz, oz);
-        const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-        const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax));
-        hr = tn <= tf;
-    }
-    const int g = (int)(b.w & 0x3fffffffu);
-    l = (b.w >> 30) & 1u ? leaf_link(g, 1) : g;
-    r = (b.w >> 31) ? leaf_link(g + 1, 1) : g + 1;
-}
-
 // Visits every leaf whose box (dilated by pad) passes `test_box`; calls
 // leaf(sorted_index) which returns false to stop.  Returns false if the
 // traversal stack overflowed.

@@ -565,34 +565,25 @@ UPBP_D void splat_camera(unsigned px, float3 c)
 // short one a few, and every accepted neighbour costs a full MIS evaluation;
 // run inside one walk per thread, both leave most lanes of a warp idle.
 //
-// range_search_kernel<kMode>: persistent warps walk a photon map's compressed
-// nodes (QNode) with one query per lane, one internal node per step; a lane
-// whose query is finished
-// takes the next one in Morton order from a global counter, so lanes stay
-// busy until the queue is empty.  A child that is a leaf is not visited: its
-// (query, primitive) pair goes into a per-warp ring in shared memory, and
-// whenever 32 pairs are waiting all lanes run the exact leaf test on one pair
-// each, so the test never runs on a partly idle warp.  Accepted pairs are
-// gathered the same way and written out 32 at a time (one atomic per 32
-// hits).  A search covers one round of the query order: once the hit list
-// is 3/4 full no lane takes a new query, the lanes finish the queries they
-// hold, and the host evaluates the list and starts the next round where this
-// one stopped.  Pairs past the capacity are dropped but still counted, and
-// such a round is repeated.
+// range_search_kernel<kMode> (upbp_range_search.cuh): persistent warps take
+// queries in processing order from a global counter and write the accepted
+// (query, neighbour) pairs to the hit list.  A search covers one round of the
+// query order: once the hit list is 3/4 full no warp takes new queries, the
+// warps finish the queries they hold, and the host evaluates the list and
+// starts the next round where this one stopped.  Pairs past the capacity are
+// dropped but still counted, and such a round is repeated.
 //
 // range_eval_kernel<kMode>: one accepted pair per thread, the records of a
-// warp's 32 pairs read together (gather_records); recomputes the pair's
-// geometry with the same predicate, evaluates the estimator with its MIS
-// weight and adds it into the camera image.
+// warp's 32 pairs read together (gather_runs, gather_records); recomputes the
+// pair's geometry with the same predicate, evaluates the estimator with its
+// MIS weight and adds it into the camera image, a run of pairs of one query at
+// once.
 enum : int { kModePb2d = 0, kModeBb1d, kModeBp2d, kRangeModes };
 template <int kMode> struct RangeMode {
     static_assert(kMode >= 0 && kMode < kRangeModes, "range-query mode");
     static constexpr bool seg = kMode != kModeBp2d;  // segment queries (else point queries)
     static constexpr bool beams = kMode != kModePb2d;  // beam map (else medium photon map)
     static constexpr int kern = kMode == kModePb2d ? kKernPb2d : kMode == kModeBb1d ? kKernBb1d : kKernBp2d;
-    // query geometry of waiting pairs in shared memory (long BB1D queries;
-    // the short PB2D and BP2D ones refill lanes too often for its flushes)
-    static constexpr bool shared_geo = kMode == kModeBb1d;
 };
 
 enum : unsigned { kQuerySurf = 1u, kQueryPp3d = 2u, kQueryBp2d = 4u };
@@ -604,33 +595,9 @@ UPBP_D const BvhView& range_map_bvh()
     return RangeMode<kMode>::beams ? p.beam_map.bvh : p.med_map.bvh;
 }
 
-constexpr int kSearchWarps = 4;
-constexpr unsigned kNoQuery = 0xffffffffu;  // no more queries in this round
-constexpr unsigned kCandRing = 128;  // > 31 waiting + 64 new pairs per step
-
-// The top kSmemStack entries of each lane's traversal stack live in shared
-// memory (column per lane, so lanes never share a bank); deeper entries go
-// to local memory.  Local memory competes with the photon maps for L1.
-constexpr int kSmemStack = 16;
-
-// A waiting pair names the lane whose query it belongs to in the top bits of
-// its leaf word (leaf indices stay below 2^kLeafShift).  With shared_geo the
-// lane's query geometry sits in shared memory, so a pair test reads only the
-// map's record from global memory; a lane then overwrites its geometry only
-// when no pair is waiting.
-constexpr unsigned kPairLeafMask = (1u << kLeafShift) - 1u;
-
-struct SearchWarp {
-    uint2 cand[kCandRing];  // (query record, map leaf | owner lane << kLeafShift)
-    uint2 hit_qb[64];
-    int stack[kSmemStack][32];
-};
-struct SearchWarpGeo : SearchWarp {
-    float4 qgeo[2][32];     // per lane: (origin, tmin), (direction, tmax)
-};
-template <int kMode>
-using SearchWarpOf = std::conditional_t<RangeMode<kMode>::shared_geo, SearchWarpGeo, SearchWarp>;
-static_assert(kLeafShift + 5 <= 32, "owner lane bits");
+}  // namespace upbp
+#include "upbp_range_search.cuh"
+namespace upbp {
 
 // The estimate of one accepted (query, neighbour) pair: the predicate's
 // geometry recomputed, the estimator with its MIS weight, added into the
@@ -638,7 +605,7 @@ static_assert(kLeafShift + 5 <= 32, "owner lane bits");
 // (segment query, or a point query's camera vertex) and of the neighbour's
 // (beam or light vertex).
 template <int kMode, bool kGuided, class FQ, class FN>
-UPBP_D void eval_range_hit(uint2 qb, FQ&& fq, FN&& fn)
+UPBP_D float3 eval_range_hit(uint2 qb, unsigned& px, FQ&& fq, FN&& fn)
 {
     using M = RangeMode<kMode>;
     const DeviceParams& p = c_params;
@@ -648,7 +615,8 @@ UPBP_D void eval_range_hit(uint2 qb, FQ&& fq, FN&& fn)
         float3 weight;
         unsigned pk, path, key;
         read_seg_query(fq, q, cw, weight, pk, path, key);
-        if (!event_kept(path, key)) return;
+        px = pk >> 8;
+        if (!event_kept(path, key)) return v3(0.f);
         float3 est;
         if constexpr (kMode == kModeBb1d) {
             Beam lb;
@@ -656,7 +624,7 @@ UPBP_D void eval_range_hit(uint2 qb, FQ&& fq, FN&& fn)
             float dist, sin_theta, t1, t2;
             if (!pred_beam_beam(q.o, q.d, q.dmin, q.dmax, lb.o, lb.d, lb.length, p.radius_bb1d_2, dist, sin_theta,
                                 t1, t2))
-                return;
+                return v3(0.f);
             float w = -1.f;
             est = p.bb1d_normalization * eval_bb1d(q, cw, lb, dist, sin_theta, t1, t2, &w, kGuided);
             UPBP_MISDBG(if (w >= 0.f) {
@@ -668,7 +636,7 @@ UPBP_D void eval_range_hit(uint2 qb, FQ&& fq, FN&& fn)
             LightVertex lv;
             read_vertex(fn, lv);
             float dist, rad2;
-            if (!pred_ray_disc(q.o, q.d, q.dmin, q.dmax, lv.hit, p.radius_pb2d_2, dist, rad2)) return;
+            if (!pred_ray_disc(q.o, q.d, q.dmin, q.dmax, lv.hit, p.radius_pb2d_2, dist, rad2)) return v3(0.f);
             float w = -1.f;
             est = p.pb2d_normalization * eval_pb2d(q, cw, lv, dist, rad2, &w, kGuided);
             UPBP_MISDBG(if (w >= 0.f) {
@@ -677,256 +645,26 @@ UPBP_D void eval_range_hit(uint2 qb, FQ&& fq, FN&& fn)
                 mis_event(e, nullptr, 0);
             });
         }
-        splat_camera(pk >> 8, weight * est);
+        return weight * est;
     } else {
         const float4 q8 = __ldg(&p.pt_queue[qb.x].q8);
+        px = fbits(q8.x);
         LightVertex cv;
         read_vertex(fq, cv);
         if (!kGuided) cv.bsdf.gcell = -1;  // the unguided instantiation has no proposal code
         Beam lb;
         read_beam(fn, lb);
         float dist, rad2;
-        if (!pred_ray_disc(lb.o, lb.d, 0.f, lb.length, cv.hit, p.radius_bp2d_2, dist, rad2)) return;
+        if (!pred_ray_disc(lb.o, lb.d, 0.f, lb.length, cv.hit, p.radius_bp2d_2, dist, rad2)) return v3(0.f);
         float w = -1.f;
-        splat_camera(fbits(q8.x),
-                     cv.thr * p.bp2d_normalization * eval_bp2d(lb, cv.path_length, cv.w, cv.bsdf, dist, rad2, &w));
+        const float3 c = cv.thr * p.bp2d_normalization * eval_bp2d(lb, cv.path_length, cv.w, cv.bsdf, dist, rad2, &w);
         UPBP_MISDBG(if (w >= 0.f) {
             MisEvent e{kMisBp2d, fbits(q8.z), cv.path_length, lb.path_idx, lb.path_length, 0u, w,
                        lb.o + lb.d * dist, cv.hit, lb.origin_offset + dist, 0.f, lb.origin_offset};
             mis_event(e, nullptr, 0);
         });
+        return c;
     }
-}
-
-// Leaf tests of the 32 (or, at the end, fewer) oldest waiting pairs, one per
-// lane; accepted pairs go to the hit buffer, which is flushed by 32.  A hit
-// is (query record, beam) or (query record, light-vertex slot).
-template <int kMode>
-UPBP_D void search_test_pairs(SearchWarpOf<kMode>& w, unsigned& head, unsigned count, unsigned& hfill, unsigned lane,
-                              unsigned& cand, unsigned& hits, unsigned long long& seen)
-{
-    const DeviceParams& p = c_params;
-    const unsigned below = (1u << lane) - 1u;
-    __syncwarp();
-    bool hit = false;
-    uint2 pr = make_uint2(0u, 0u);
-    unsigned id = 0;
-    if (lane < count) {
-        pr = w.cand[(head + lane) % kCandRing];
-        const unsigned leaf = pr.y & kPairLeafMask, owner = pr.y >> kLeafShift;
-        if constexpr (RangeMode<kMode>::seg) {
-            const float4* r = p.seg_queue[pr.x].q;
-            float4 q0, q1;
-            if constexpr (RangeMode<kMode>::shared_geo) {
-                q0 = w.qgeo[0][owner];
-                q1 = w.qgeo[1][owner];
-            } else {
-                q0 = __ldg(&r[0]);
-                q1 = __ldg(&r[1]);
-            }
-            if constexpr (kMode == kModeBb1d) {
-                BeamSegHit h;
-                hit = beam_chunk_vs_segment(p.beam_map, (int)leaf, xyz(q0), xyz(q1), q0.w, q1.w, p.radius_bb1d_2,
-                                            false, p.do_bp2d != 0, -1, &r[2], cand, h);
-                id = h.beam;
-            } else {
-                const float4 pp = __ldg(&p.med_map.pos[leaf]);
-                float dist, rad2;
-                cand++;
-                hit = pred_ray_disc(xyz(q0), xyz(q1), q0.w, q1.w, xyz(pp), p.radius_pb2d_2, dist, rad2);
-                id = fbits(pp.w);
-            }
-        } else {
-            // BP2D: beams_near_point's leaf test, the chunk holding the
-            // beam's closest point reports it
-            const float3 x = xyz(__ldg(&p.pt_queue[pr.x].v.q[0]));
-            const float4 s0 = __ldg(&p.beam_map.seg[3 * leaf]), s1 = __ldg(&p.beam_map.seg[3 * leaf + 1]);
-            float dist, rad2;
-            cand++;
-            if (pred_ray_disc(xyz(s0), xyz(s1), 0.f, s0.w, x, p.radius_bp2d_2, dist, rad2)) {
-                const float4 s2 = __ldg(&p.beam_map.seg[3 * leaf + 2]);  // the chunk's range, for accepted pairs only
-                hit = dist >= s2.x && dist < s2.y;
-            }
-            id = fbits(s1.w) & 0x7fffffffu;
-        }
-    }
-    head += count;
-    const unsigned hm = __ballot_sync(~0u, hit);
-    if (hit) {
-        const unsigned pos = hfill + __popc(hm & below);
-        w.hit_qb[pos] = make_uint2(pr.x, id);
-        hits++;
-    }
-    hfill += __popc(hm);
-    if (hfill >= 32) {
-        __syncwarp();
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&p.hit_state->total, 32ull);
-        base = __shfl_sync(~0u, base, 0);
-        seen = base + 32;
-        if (base + lane < p.hit_capacity) p.hit_qb[base + lane] = w.hit_qb[lane];
-        __syncwarp();
-        if (lane + 32 < hfill) w.hit_qb[lane] = w.hit_qb[lane + 32];
-        hfill -= 32;
-    }
-    __syncwarp();
-}
-
-template <int kMode>
-__global__ void __launch_bounds__(128) range_search_kernel(int slot)
-{
-    using M = RangeMode<kMode>;
-    begin_kernel(M::kern, slot);
-    const DeviceParams& p = c_params;
-    __shared__ SearchWarpOf<kMode> s_warp[kSearchWarps];
-    SearchWarpOf<kMode>& w = s_warp[threadIdx.x >> 5];
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    // this round's range of the processing order, within the queue
-    const unsigned nq = M::seg ? min(p.queue_count[0], p.seg_capacity) : min(p.queue_count[1], p.pt_capacity);
-    const unsigned n = min(p.query_end, nq) - min(p.query_begin, min(p.query_end, nq));
-    unsigned long long seen = 0;  // hit total after this warp's last flush
-    const BvhView bvh = range_map_bvh<kMode>();
-    int node = kWalkDone, sp = 0;
-    int deep[kStackDepth - kSmemStack];
-    float3 inv = v3(0.f), oinv = v3(0.f), x = v3(0.f);
-    float tmin = 0.f, tmax = 0.f;
-    unsigned qk = 0;
-    bool exhausted = false;  // no queries left for this warp (the same in every lane)
-    bool overflow = false;
-    unsigned head = 0, tail = 0, hfill = 0;  // same values in every lane
-    unsigned visits = 0, cand = 0, hits = 0;
-    for (;;) {
-        // primitives of the leaf children reached this step (a compressed
-        // node's leaves hold one primitive each), -1 for none
-        int leaf0 = -1, leaf1 = -1;
-        const unsigned idle = __ballot_sync(~0u, node == kWalkDone);
-        if (exhausted && idle == ~0u) break;
-        const unsigned want = exhausted ? 0u : idle;
-        if (want) {
-            // a lane that takes a new query overwrites its geometry: test the
-            // pairs still waiting first
-            if (M::shared_geo && tail != head)
-                search_test_pairs<kMode>(w, head, tail - head, hfill, lane, cand, hits, seen);
-            // no new queries once the hit list is 3/4 full, as far as this
-            // warp saw at its last flush of hits (no extra load of the
-            // counter, which every flush and request updates)
-            const int leader = __ffs(want) - 1;
-            unsigned base = kNoQuery;
-            if ((int)lane == leader && seen < p.hit_soft_limit)
-                base = atomicAdd(&p.hit_state->fetched, (unsigned)__popc(want));
-            base = __shfl_sync(~0u, base, leader);
-            // the queue is used up once a lane's index falls past its end
-            if (base == kNoQuery || base + (unsigned)__popc(want) > n) exhausted = true;
-            if ((want >> lane) & 1u) {
-                const unsigned r = base + __popc(want & below);
-                bool take = base != kNoQuery && r < n;
-                const unsigned j = p.query_begin + r;
-                if (take) {
-                    if constexpr (M::seg) {
-                        qk = p.seg_order ? __ldg(&p.seg_order[j]) : j;
-                        const float4* r = p.seg_queue[qk].q;
-                        const float4 q0 = __ldg(&r[0]), q1 = __ldg(&r[1]);
-                        tmin = q0.w;
-                        tmax = q1.w;
-                        inv = safe_inv(xyz(q1));
-                        oinv = oinv_of(xyz(q0), inv);
-                        if constexpr (M::shared_geo) {
-                            w.qgeo[0][lane] = q0;
-                            w.qgeo[1][lane] = q1;
-                        }
-                    } else {
-                        // point queries of other estimators, or of camera paths
-                        // that failed earlier, are skipped
-                        qk = p.pt_order ? __ldg(&p.pt_order[j]) : j;
-                        const float4 q8 = __ldg(&p.pt_queue[qk].q8);
-                        take = (fbits(q8.y) & kQueryBp2d) && event_kept(fbits(q8.z), fbits(q8.w));
-                        x = xyz(__ldg(&p.pt_queue[qk].v.q[0]));
-                    }
-                }
-                if (take) {
-                    sp = 0;
-                    node = bvh.count > 1 ? 0 : kWalkDone;
-                    if (bvh.count == 1) {  // a one-leaf map
-                        leaf0 = 0;
-                    }
-                }
-            }
-        }
-        if (node != kWalkDone) {
-            // one internal node: leaf children become pairs, internal ones are visited
-            visits++;
-            bool hl, hr;
-            int cl, cr;
-            if constexpr (M::seg) {
-                qnode_slab(bvh.qnodes, node, inv, oinv, tmin, tmax, hl, hr, cl, cr);
-            } else {
-                const NodeBoxes nb = load_qnode(bvh.qnodes, node);
-                hl = inside(nb.llo, nb.lhi, x);
-                hr = inside(nb.rlo, nb.rhi, x);
-                cl = nb.l;
-                cr = nb.r;
-            }
-            int next = -1, other = -1;
-            if (hl) {
-                if (cl < 0) {
-                    leaf0 = leaf_first(cl);
-                } else {
-                    next = cl;
-                }
-            }
-            if (hr) {
-                if (cr < 0) {
-                    leaf1 = leaf_first(cr);
-                } else if (next < 0) {
-                    next = cr;
-                } else {
-                    other = cr;
-                }
-            }
-            if (other >= 0) {
-                if (sp < kSmemStack)
-                    w.stack[sp++][lane] = other;
-                else if (sp < kStackDepth)
-                    deep[sp++ - kSmemStack] = other;
-                else
-                    overflow = true;
-            }
-            if (next >= 0) {
-                node = next;
-            } else if (sp > 0) {
-                --sp;
-                node = sp < kSmemStack ? w.stack[sp][lane] : deep[sp - kSmemStack];
-            } else {
-                node = kWalkDone;
-            }
-        }
-        // each reached leaf becomes a waiting pair (a lane adds up to two,
-        // next to each other); 32 waiting pairs are tested at once.  The
-        // walk tests compressed boxes, which contain the exact ones: the leaf
-        // test re-checks a chunk's own box where it matters.
-        {
-            const unsigned m0 = __ballot_sync(~0u, leaf0 >= 0), m1 = __ballot_sync(~0u, leaf1 >= 0);
-            unsigned at = tail + __popc(m0 & below) + __popc(m1 & below);
-            if (leaf0 >= 0) w.cand[at++ % kCandRing] = make_uint2(qk, (unsigned)leaf0 | (lane << kLeafShift));
-            if (leaf1 >= 0) w.cand[at % kCandRing] = make_uint2(qk, (unsigned)leaf1 | (lane << kLeafShift));
-            tail += __popc(m0) + __popc(m1);
-#pragma unroll 1
-            while (tail - head >= 32) search_test_pairs<kMode>(w, head, 32, hfill, lane, cand, hits, seen);
-        }
-    }
-    if (tail != head) search_test_pairs<kMode>(w, head, tail - head, hfill, lane, cand, hits, seen);
-    __syncwarp();
-    if (hfill) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&p.hit_state->total, (unsigned long long)hfill);
-        base = __shfl_sync(~0u, base, 0);
-        if (lane < hfill && base + lane < p.hit_capacity) p.hit_qb[base + lane] = w.hit_qb[lane];
-    }
-    count_work(kCtrNodes, visits);
-    count_work(M::beams ? kCtrBeamCand : kCtrPointCand, cand);
-    count_work(M::beams ? kCtrBeamHit : kCtrPointHit, hits);
-    if (overflow) flag_status(kErrTraversalStack);
 }
 
 // The 128-byte records of a warp's 32 hits, read together: eight lanes load
@@ -951,8 +689,25 @@ UPBP_D void gather_records(const float4* rec, float4 (&out)[8], float4 (*s)[9], 
     for (int i = 0; i < 8; i++) out[i] = s[lane][i];
 }
 
-// One warp per 32 consecutive hits; lanes past the end read the warp's
-// first hit's records and evaluate nothing.
+// The query records of a warp's 32 hits: consecutive hits mostly share their
+// query (the search finds a query's pairs side by side), so a record is
+// loaded once per run of equal queries, four records at a time, and its
+// lanes read the run's row.  `run` is the lane's run, `runs` their number.
+UPBP_D void gather_runs(const float4* rec, unsigned run, unsigned heads, float4 (&out)[8], float4 (*s)[9],
+                        const float4** first, unsigned lane)
+{
+    const unsigned runs = __popc(heads);
+    __syncwarp();
+    if ((heads >> lane) & 1u) first[run] = rec;
+    __syncwarp();
+    for (unsigned r = lane >> 3; r < runs; r += 4) s[r][lane & 7u] = __ldg(first[r] + (lane & 7u));
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; i++) out[i] = s[run][i];
+}
+
+// One warp per 32 consecutive hits.  The estimates of a run of hits of one
+// query are summed over its lanes and added to the image once.
 // kGuided: a learned-proposal table is in use (the unguided instantiation,
 // the common case, contains none of the proposal's code).
 template <int kMode, bool kGuided>
@@ -962,12 +717,25 @@ __global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
     begin_kernel(M::kern, slot);
     const DeviceParams& p = c_params;
     __shared__ float4 s_rec[kEvalWarps][32][9];
+    __shared__ const float4* s_first[kEvalWarps][32];
     float4(*s)[9] = s_rec[threadIdx.x >> 5];
+    const float4** first = s_first[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned n = (unsigned)min(p.hit_state->total, (unsigned long long)p.hit_capacity);
     for (unsigned base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
-        const unsigned j = base + lane;
-        const uint2 qb = __ldg(&p.hit_qb[j < n ? j : base]);
+        // lanes past the end or on an empty slot join the run before them (or
+        // the first hit's) and evaluate nothing
+        uint2 qb = base + lane < n ? __ldcs(&p.hit_qb[base + lane]) : make_uint2(kNoHit, 0u);
+        const unsigned full = __ballot_sync(~0u, qb.x != kNoHit);
+        if (!full) continue;
+        const bool valid = qb.x != kNoHit;
+        const unsigned upto = full & (0xffffffffu >> (31u - lane));
+        const int src = upto ? 31 - __clz(upto) : __ffs(full) - 1;
+        qb.x = __shfl_sync(~0u, qb.x, src);
+        qb.y = __shfl_sync(~0u, qb.y, src);
+        const unsigned before = __shfl_up_sync(~0u, qb.x, 1);
+        const unsigned heads = __ballot_sync(~0u, lane == 0 || qb.x != before);
+        const unsigned run = __popc(heads & (0xffffffffu >> (31u - lane))) - 1u;
         const float4* qrec;
         const float4* nrec;
         if constexpr (M::seg)
@@ -979,9 +747,24 @@ __global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
         else
             nrec = p.vertices[qb.y].q;
         float4 qa[8], na[8];
-        gather_records(qrec, qa, s, lane);
+        gather_runs(qrec, run, heads, qa, s, first, lane);
         gather_records(nrec, na, s, lane);
-        if (j < n) eval_range_hit<kMode, kGuided>(qb, [&](int i) { return qa[i]; }, [&](int i) { return na[i]; });
+        float3 c = v3(0.f);
+        unsigned px = 0xffffffu;
+        if (valid)
+            c = eval_range_hit<kMode, kGuided>(qb, px, [&](int i) { return qa[i]; }, [&](int i) { return na[i]; });
+        // sums over the lanes of each run, left in its first lane
+        const unsigned next = lane == 31u ? 0u : heads & (~0u << (lane + 1u));
+        const unsigned last = next ? (unsigned)__ffs(next) - 2u : 31u;  // last lane of this lane's run
+#pragma unroll
+        for (unsigned d = 1; d < 32; d *= 2) {
+            const float x = __shfl_down_sync(~0u, c.x, d), y = __shfl_down_sync(~0u, c.y, d),
+                        z = __shfl_down_sync(~0u, c.z, d);
+            if (lane + d <= last) c = c + make_float3(x, y, z);
+        }
+        // (a run may begin with empty lanes: only before the first hit)
+        px = __shfl_sync(~0u, px, max(31 - __clz(heads & (0xffffffffu >> (31u - lane))), __ffs(full) - 1));
+        if ((heads >> lane) & 1u) splat_camera(px, c);
     }
 }
 
@@ -1444,27 +1227,30 @@ __global__ void __launch_bounds__(256) k_resolve_camera(int slot)
     }
 }
 
-// Morton keys of the query records (segment midpoint / vertex position in
-// the scene's bounding cube), so the query kernels walk spatially coherent
-// warps through the photon maps.
+// Morton keys of the query records in the scene's bounding cube, so that
+// queries a warp takes together lie close together: of a segment both ends
+// (30 bits each, interleaved: neighbours by midpoint alone may cross at any
+// angle), of a point query its position.
 template <bool kSeg>
-__global__ void k_query_keys(int slot, unsigned n, unsigned* keys, unsigned* vals)
+__global__ void k_query_keys(int slot, unsigned n, unsigned long long* keys64, unsigned* keys, unsigned* vals)
 {
     begin_kernel(kKernCameraExtend, slot);
     const DeviceParams& p = c_params;
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    float3 x;
+    const float inv = .5f / p.scene_radius;
+    auto code = [&](float3 x) { return morton3((x - p.scene_center) * inv + v3(.5f)); };
     if (kSeg) {
         const float4 q0 = p.seg_queue[k].q[0], q1 = p.seg_queue[k].q[1];
-        const float t = q1.w < 1e30f ? .5f * (q0.w + q1.w) : q0.w;
-        x = xyz(q0) + xyz(q1) * t;
+        // both ends, the far one of an open segment taken at the scene's size
+        const float t1 = fminf(q1.w, q0.w + 2.f * p.scene_radius);
+        const unsigned a = code(xyz(q0) + xyz(q1) * q0.w), b = code(xyz(q0) + xyz(q1) * t1);
+        unsigned long long key = 0;
+        for (int l = 9; l >= 0; l--) key = key << 6 | ((a >> 3 * l) & 7u) << 3 | ((b >> 3 * l) & 7u);
+        keys64[k] = key;
     } else {
-        x = xyz(p.pt_queue[k].v.q[0]);
+        keys[k] = code(xyz(p.pt_queue[k].v.q[0]));
     }
-    const float inv = .5f / p.scene_radius;
-    const float3 u = (x - p.scene_center) * inv + v3(.5f);
-    keys[k] = morton3(u);
     vals[k] = k;
 }
 

@@ -255,8 +255,9 @@ struct upbp_ctx {
     double* d_acc = nullptr;
     unsigned* d_status = nullptr;
     BvhNode *d_surf_nodes = nullptr, *d_med_nodes = nullptr, *d_beam_nodes = nullptr;
-    QNode *d_med_qnodes = nullptr, *d_beam_qnodes = nullptr;  // compressed copies for the range searches
-    float4 *d_surf_pos = nullptr, *d_med_pos = nullptr, *d_beam_seg = nullptr;
+    QNode4 *d_med_qnodes = nullptr, *d_beam_qnodes = nullptr;  // compressed copies for the range searches
+    float4 *d_surf_pos = nullptr, *d_med_pos = nullptr;
+    uint2* d_beam_leaf = nullptr;  // the beam map's leaves: BeamMap::chunk
     unsigned *d_chunk_counts = nullptr, *d_chunk_offsets = nullptr;
     uint2* d_chunks = nullptr;
     unsigned chunk_capacity = 0;
@@ -873,14 +874,20 @@ float relative_radius(float r, float scene_radius) { return r < 0.f ? -r * scene
 int ensure_sort(upbp_ctx* c, int q, unsigned n)
 {
     if (n <= c->sort_capacity[q]) return UPBP_OK;
-    for (auto& b : c->d_sort[q]) {
-        cudaFree(b);
-        UPBP_CK(dalloc(&b, n));
+    for (int k = 0; k < 4; k++) {
+        cudaFree(c->d_sort[q][k]);
+        UPBP_CK(dalloc(&c->d_sort[q][k], q == 0 && k < 2 ? 2 * (size_t)n : n));  // segment keys: 64 bits
     }
     c->sort_capacity[q] = n;
     cub::DoubleBuffer<unsigned> kb(c->d_sort[q][0], c->d_sort[q][1]), vb(c->d_sort[q][2], c->d_sort[q][3]);
     size_t bytes = 0;
-    UPBP_CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, (int)n, 0, 30));
+    if (q == 0) {
+        cub::DoubleBuffer<unsigned long long> kb64((unsigned long long*)c->d_sort[0][0],
+                                                   (unsigned long long*)c->d_sort[0][1]);
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb64, vb, (int)n, 0, 60));
+    } else {
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, (int)n, 0, 30));
+    }
     if (bytes > c->sort_temp_bytes) {
         cudaFree(c->d_sort_temp);
         UPBP_CK(cudaMalloc(&c->d_sort_temp, bytes));
@@ -896,14 +903,18 @@ int sort_queries(upbp_ctx* c, int q, unsigned n, const unsigned** order)
     if (n < 2) return UPBP_OK;
     if (ensure_sort(c, q, n) != UPBP_OK) return UPBP_ERR_CUDA;
     unsigned** b = c->d_sort[q];
-    if (q == 0)
-        PK(c).query_keys[1]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, b[0], b[2]);
-    else
-        PK(c).query_keys[0]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, b[0], b[2]);
-    UPBP_CK(cudaGetLastError());
     cub::DoubleBuffer<unsigned> kb(b[0], b[1]), vb(b[2], b[3]);
     size_t tb = c->sort_temp_bytes;
-    UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb, vb, (int)n, 0, 30, c->st));
+    if (q == 0) {
+        cub::DoubleBuffer<unsigned long long> kb64((unsigned long long*)b[0], (unsigned long long*)b[1]);
+        PK(c).query_keys[1]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, kb64.Current(), nullptr, b[2]);
+        UPBP_CK(cudaGetLastError());
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb64, vb, (int)n, 0, 60, c->st));
+    } else {
+        PK(c).query_keys[0]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, nullptr, b[0], b[2]);
+        UPBP_CK(cudaGetLastError());
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb, vb, (int)n, 0, 30, c->st));
+    }
     *order = vb.Current();
     return UPBP_OK;
 }
@@ -917,11 +928,11 @@ int ensure_chunks(upbp_ctx* c, unsigned n)
         cudaFree(c->d_chunks);
         cudaFree(c->d_beam_nodes);
         cudaFree(c->d_beam_qnodes);
-        cudaFree(c->d_beam_seg);
+        cudaFree(c->d_beam_leaf);
         UPBP_CK(dalloc(&c->d_chunks, cap));
         UPBP_CK(dalloc(&c->d_beam_nodes, cap));
         UPBP_CK(dalloc(&c->d_beam_qnodes, cap));
-        UPBP_CK(dalloc(&c->d_beam_seg, 3 * (size_t)cap));
+        UPBP_CK(dalloc(&c->d_beam_leaf, cap));
         c->chunk_capacity = cap;
     }
     if (cap > c->sc.capacity) {
@@ -930,6 +941,23 @@ int ensure_chunks(upbp_ctx* c, unsigned n)
         if (alloc_scratch(c->sc, cap) != UPBP_OK) return UPBP_ERR_CUDA;
     }
     return UPBP_OK;
+}
+
+// How a range search splits its queries.  Larger units share more of their
+// walks (groups), smaller ones spread uneven queries over the warps: BB1D,
+// whose queries cost a thousand node tests each, takes units of at most 8 and
+// a quarter of a warp's even share (box 256x256 11.4 ms; 12.1 at an eighth,
+// 13.3 at a half; dense beams 43.6 ms; 52.9 with units of up to 32); the
+// short PB2D and BP2D queries share more (media field PB2D 1.6 ms, 1.9 with
+// units of 8).  A group's start or end points stay within `spread` of the
+// query radius: BB1D 4 (media field 18.2 ms; 18.5 at 6, 20.2 at 10), where
+// the tests of leaves outside a query's own reach begin to cost more than the
+// shared nodes save; the point maps' smaller boxes and cheaper tests 6.
+void range_search_split(DeviceParams& P, int mode)
+{
+    P.unit_max = mode == kModeBb1d ? 8u : 32u;
+    P.units_per_warp = mode == kModeBb1d ? 4u : 3u;
+    P.group_spread = mode == kModeBb1d ? 4.f * P.rad_beam : 6.f * (mode == kModePb2d ? P.rad_point_med : P.rad_beam);
 }
 
 // Largest range-query hit list (8 bytes per entry, 34 GB, allocated only
@@ -1504,7 +1532,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
         // beam-map boxes: the beam radius (BB1D and BP2D), the box tests' rounding
         // and the BB1D predicate's t1 error on nearly parallel lines
         const float beam_dilate = P.rad_beam * 1.0001f + P.beam_cull_eps;
-        P.beam_map = BeamMap{BvhView{c->d_beam_nodes, 0, c->d_beam_qnodes}, c->d_beam_seg, beam_dilate};
+        P.beam_map = BeamMap{BvhView{c->d_beam_nodes, 0, c->d_beam_qnodes}, c->d_beam_leaf, c->d_beams, beam_dilate};
         if (P.build_surf && ns > 0) {
             BoxSource src{};
             src.kind = 1;
@@ -1543,7 +1571,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             UPBP_CK(cudaStreamSynchronize(c->st));
             const unsigned nchunks = tail[0] + tail[1];
             if (ensure_chunks(c, nchunks) != UPBP_OK) return UPBP_ERR_CUDA;
-            P.beam_map = BeamMap{BvhView{c->d_beam_nodes, 0, c->d_beam_qnodes}, c->d_beam_seg, beam_dilate};
+            P.beam_map = BeamMap{BvhView{c->d_beam_nodes, 0, c->d_beam_qnodes}, c->d_beam_leaf, c->d_beams, beam_dilate};
             k_chunk_expand<<<(nb + 255) / 256, 256, 0, c->st>>>(c->d_chunk_counts, c->d_chunk_offsets, nb, c->d_chunks);
             BoxSource src{};
             src.kind = 3;
@@ -1572,7 +1600,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 UPBP_CK(build_lbvh(src, nchunks, c->d_beam_nodes, c->sc, c->st, &order));
             }
             k_gather_chunks<<<(nchunks + 255) / 256, 256, 0, c->st>>>(c->d_chunks, c->d_beams, order, nchunks,
-                                                                      P.bb1d_used_light_subpath_count, c->d_beam_seg);
+                                                                      P.bb1d_used_light_subpath_count, c->d_beam_leaf);
             if (nchunks > 1)
                 k_quantize<<<(nchunks - 1 + 255) / 256, 256, 0, c->st>>>(c->d_beam_nodes, (int)nchunks - 1,
                                                                          c->d_beam_qnodes);
@@ -1657,7 +1685,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 const unsigned* order = nullptr;
                 UPBP_CK(build_lbvh(c->ploc_src, n, c->d_beam_nodes, c->sc, c->st, &order));
                 k_gather_chunks<<<(n + 255) / 256, 256, 0, c->st>>>(c->d_chunks, c->d_beams, order, n,
-                                                                    P.bb1d_used_light_subpath_count, c->d_beam_seg);
+                                                                    P.bb1d_used_light_subpath_count, c->d_beam_leaf);
                 k_quantize<<<(n - 1 + 255) / 256, 256, 0, c->st>>>(c->d_beam_nodes, (int)n - 1, c->d_beam_qnodes);
                 launches += 7;
             }
@@ -1730,6 +1758,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 P.hit_soft_limit = c->hit_capacity - c->hit_capacity / 4;
                 P.query_begin = begin;
                 P.query_end = end;
+                range_search_split(P, mode);
                 h2d += sizeof(P);
                 UPBP_CK(upload_params(c));
                 const int g = (int)cap_grid(c, (unsigned)c->search_grid[mode]);
@@ -2461,7 +2490,7 @@ extern "C" void upbp_destroy(upbp_ctx* c)
                     c->d_env_img, c->d_env_dist, c->d_env_row_int, c->real.spheres, c->real.sph_mat, c->imag.spheres, c->imag.sph_mat,
                     c->imag.nodes, c->imag.tri, c->imag.normals, c->imag.record, c->d_vertices, c->d_path_count,
                     c->d_counters, c->d_idx_s, c->d_idx_m, c->d_beams, c->d_fb, c->d_acc, c->d_status,
-                    c->d_surf_nodes, c->d_med_nodes, c->d_beam_nodes, c->d_med_qnodes, c->d_beam_qnodes, c->d_surf_pos, c->d_med_pos, c->d_beam_seg,
+                    c->d_surf_nodes, c->d_med_nodes, c->d_beam_nodes, c->d_med_qnodes, c->d_beam_qnodes, c->d_surf_pos, c->d_med_pos, c->d_beam_leaf,
                     c->d_chunk_counts, c->d_chunk_offsets, c->d_chunks, c->d_scan_temp, c->d_work,
                     c->d_qcount, c->d_conn, c->d_nee, c->d_bpt, c->d_nee_color, c->d_bpt_color,
                     c->d_path_err, c->d_path_color, c->d_hit_state, c->d_work_saved, c->d_hit_qb, c->d_cam_fb, c->d_seg_queue, c->d_pt_queue, c->d_sort[0][0], c->d_sort[0][1],

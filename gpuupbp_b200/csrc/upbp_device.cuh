@@ -106,36 +106,29 @@ UPBP_HD int leaf_link(int first, int count) { return ~(first | ((count - 1) << k
 UPBP_HD int leaf_first(int link) { return (~link) & ((1 << kLeafShift) - 1); }
 UPBP_HD int leaf_count(int link) { return ((~link) >> kLeafShift) + 1; }
 
-// Compressed two-wide node of a photon map, 32 bytes (half a BvhNode), for
-// the range searches, which were bound by the L1's lookups (lanes of a warp
-// read nodes at unrelated addresses and each lane's 16-byte part of a load is
-// looked up separately; the path kernels, bound by divergence, stay on
-// BvhNodes, where decoding cost more than it saved): the node's box
-// origin and a power-of-two step per axis, both children's boxes as 8-bit
-// multiples of the step (lower planes rounded down, upper planes up, with
-// the decoder's own arithmetic, so each stored box contains the exact one),
-// and the children of a Karras hierarchy of one-primitive leaves, which are
-// always gamma and gamma + 1: link = gamma | left-is-leaf << 30 |
-// right-is-leaf << 31.
-struct __align__(32) QNode {
+// Compressed four-wide node of a photon map, 48 bytes, for the range
+// searches: the grandchildren of a binary node (a child that is a leaf stays
+// one child).  The node's box origin and a power-of-two step per axis, the
+// children's boxes as 8-bit multiples of the step (lower planes rounded
+// down, upper planes up, with the decoder's own arithmetic, so each stored box
+// contains the exact one), and two links: the children of a binary node are
+// always gamma and gamma + 1, so one index names both.
+struct __align__(16) QNode4 {
     float4 a;  // origin.xyz; w: biased step exponents x | y << 8 | z << 16
-    uint4 b;   // plane bytes: left lo xyz, left hi xyz, right lo xyz, right hi xyz; w: link
+    uint4 b;   // plane bytes, two children a word (lo, hi, lo, hi): x planes, x planes, y, y
+    uint4 c;   // x, y: z planes; z: link of children 0, 1; w: of children 2, 3
 };
+// Link bits beside the index: which of its two children are leaves, or that
+// it is a single leaf.
+enum : unsigned { kQnodeLeaf0 = 1u << 28, kQnodeLeaf1 = 1u << 29, kQnodeSingle = 1u << 30 };
 
 // Step 2^(e - 127) of a biased exponent byte e in 1..254.
 UPBP_D float qnode_step(unsigned e) { return __uint_as_float(e << 23); }
 
-// Plane `byte` of a QNode word: origin + q * step with q the byte (the one
-// rounding of the decoder; the encoder checks its bytes with it).
-UPBP_D float qnode_plane(unsigned word, int byte, float step, float origin)
-{
-    return __fmaf_rn((float)((word >> (8 * byte)) & 0xffu), step, origin);
-}
-
 struct BvhView {
     const BvhNode* nodes;
     unsigned count;          // primitives
-    const QNode* qnodes;     // the same hierarchy compressed (photon maps), or nullptr
+    const QNode4* qnodes;     // the same hierarchy compressed (photon maps), or nullptr
 };
 
 // Triangles in BVH leaf order: v0 (w = original index bits), e1, e2.
@@ -226,12 +219,13 @@ struct PointMap {
 };
 
 // Beam map: BVH over beam chunks (sub-segments of each beam) in leaf order.
-//   seg[3i] = (origin.xyz, length), seg[3i+1] = (direction.xyz, beam index bits),
-//   seg[3i+2] = (t0, t1) of the beam chunk this leaf covers, beam medium id
-//   bits, chunk index | chunk count << 16 bits
+//   chunk[i] = (beam index | BB1D-eligible << 31, chunk index | chunk count << 16);
+//   the beam's own line is read from the first 32 bytes of its record.  (A
+//   48-byte copy per leaf made a map of 1.9M chunks larger than the L2.)
 struct BeamMap {
     BvhView bvh;
-    const float4* seg;
+    const uint2* chunk;
+    const BeamRec* beams;
     float dilate;  // the leaf boxes' dilation (BoxSource.dilate of the build)
 };
 
@@ -400,6 +394,8 @@ struct DeviceParams {
     uint2* hit_qb;                    // (query record index, beam index or light-vertex slot)
     unsigned hit_capacity;
     unsigned query_begin, query_end;
+    unsigned unit_max, units_per_warp;  // queries a warp takes at once (range_search_split)
+    float group_spread;               // largest box of a group's start or end points
     unsigned long long hit_soft_limit;
     HitState* hit_state;
 

@@ -10,7 +10,7 @@
 namespace upbp_kernels {
 
 using SlotKernel = void (*)(int);
-using KeyKernel = void (*)(int, unsigned, unsigned*, unsigned*);
+using KeyKernel = void (*)(int, unsigned, unsigned long long*, unsigned*, unsigned*);
 
 constexpr int kModes = 3;  // PB2D, BB1D, BP2D range modes
 

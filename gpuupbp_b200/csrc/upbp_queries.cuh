@@ -82,38 +82,32 @@ UPBP_D bool chunk_reached(float3 bo, float3 bd, float len, unsigned k, unsigned 
 }
 
 // The BB1D test of one beam-map leaf against a query segment: the path mask,
-// the medium filter and the exact beam-beam predicate, which looks at the
-// whole beam, so every chunk of an accepted beam passes it; one of them
-// reports the beam.  That is the chunk holding the beam's closest point t2
-// when the walk reaches its box.  The predicate's t2 can be far from the
-// true closest point (it divides by d1.d2, which is tiny for nearly
+// the exact beam-beam predicate, which looks at the whole beam, so every
+// chunk of an accepted beam passes it, and the medium filter; one of the
+// chunks reports the beam.  That is the chunk holding the beam's closest
+// point t2 when the query reaches its box.  The predicate's t2 can be far
+// from the true closest point (it divides by d1.d2, which is tiny for nearly
 // perpendicular lines), and then the chunk holding it can lie outside the
 // query's reach: in that case the first chunk of the beam whose box the query
 // reaches reports instead (a check that is only needed when the computed
-// closest points are far apart).  A chunk whose own box passes the walk's box test
-// is always visited, so exactly one chunk reports each accepted beam, and
-// the set equals a test of every beam (a chunk reached only as part of a
-// leaf of several chunks never reports).  cand counts the leaves that reach
-// the predicate; own_box tells that the walk reached this chunk through a
-// leaf of its own (so its box passed).  The query's medium is `med`, or,
-// when med_src is set, med_src->w: read, like the chunk's medium and range,
-// only for pairs the predicate accepts (three of four are rejected, and each
-// record read is one more L1 lookup per lane).
+// closest points are far apart).  A walk tests at least the chunks whose
+// boxes the query reaches, so exactly one chunk reports each accepted beam,
+// and the set equals a test of every beam, however many further chunks the
+// walk tests.  cand counts the leaves that reach the predicate.
 UPBP_D bool beam_chunk_vs_segment(const BeamMap& map, int i, float3 o, float3 d, float tmin, float tmax, float r2,
-                                  bool own_box, bool need_mask, int med, const float4* med_src, unsigned& cand,
-                                  BeamSegHit& h)
+                                  bool need_mask, int med, unsigned& cand, BeamSegHit& h)
 {
-    const float4 s1 = __ldg(&map.seg[3 * i + 1]);
-    const unsigned bits = fbits(s1.w);
+    const uint2 ch = __ldg(&map.chunk[i]);
+    const unsigned bits = ch.x;
     if (need_mask && !(bits >> 31)) return false;
-    const float4 s0 = __ldg(&map.seg[3 * i]);
+    const BeamRec* beam = map.beams + (bits & 0x7fffffffu);
+    const float4 s0 = __ldg(&beam->q[0]), s1 = __ldg(&beam->q[1]);
     cand++;
     if (!pred_beam_beam(o, d, tmin, tmax, xyz(s0), xyz(s1), s0.w, r2, h.dist, h.sin_theta, h.t1, h.t2)) return false;
-    const float4 s2 = __ldg(&map.seg[3 * i + 2]);
-    if (med_src) med = (int)fbits(__ldg(med_src).w);
-    if (med >= 0 && (int)fbits(s2.z) != med) return false;
+    if (med >= 0 && (int)fbits(s1.w) != med) return false;
     h.beam = bits & 0x7fffffffu;
-    const bool mine = h.t2 >= s2.x && h.t2 < s2.y;
+    const unsigned k = ch.y & 0xffffu, n = ch.y >> 16;
+    const bool mine = h.t2 >= chunk_t(s0.w, k, n) && h.t2 < chunk_t(s0.w, k + 1, n);
     const float3 bo = xyz(s0), bd = xyz(s1);
     // Usual case: the computed closest points lie within the dilation of each
     // other (less a rounding margin), so the query passes through the dilated
@@ -121,10 +115,9 @@ UPBP_D bool beam_chunk_vs_segment(const BeamMap& map, int i, float3 o, float3 d,
     const float3 gap = (o + d * h.t1) - (bo + bd * h.t2);
     const float inner = map.dilate - 2.f * c_params.cull_eps;
     if (inner > 0.f && dot(gap, gap) <= inner * inner) return mine;
-    const unsigned kc = fbits(s2.w), k = kc & 0xffffu, n = kc >> 16;
-    // a leaf of several chunks is visited when any of its chunks is in
-    // reach, so this chunk's own box decides, as for every other chunk
-    if (!own_box && !chunk_reached(bo, bd, s0.w, k, n, map.dilate, o, d, tmin, tmax)) return false;
+    // a walk may test a chunk out of the query's reach, so its own box
+    // decides, as for every other chunk
+    if (!chunk_reached(bo, bd, s0.w, k, n, map.dilate, o, d, tmin, tmax)) return false;
     if (mine) return true;
     if (chunk_reached(bo, bd, s0.w, chunk_of(h.t2, s0.w, n), n, map.dilate, o, d, tmin, tmax)) return false;
     for (unsigned j = 0; j < k; j++)
@@ -146,7 +139,7 @@ UPBP_D void beams_near_segment(const BeamMap& map, float3 o, float3 d, float tmi
             s, map.bvh, [&](float3 lo, float3 hi) { return slab(lo, hi, inv, oinv, tmin, tmax); }, overflow, visits);
         BeamSegHit h;
         if (leaf >= 0 &&
-            beam_chunk_vs_segment(map, leaf, o, d, tmin, tmax, r2, false, need_mask, med, nullptr, cand, h)) {
+            beam_chunk_vs_segment(map, leaf, o, d, tmin, tmax, r2, need_mask, med, cand, h)) {
             hits++;
             f(h.beam, h.dist, h.sin_theta, h.t1, h.t2);
         }
@@ -155,6 +148,18 @@ UPBP_D void beams_near_segment(const BeamMap& map, float3 o, float3 d, float tmi
     count_work(kCtrBeamCand, cand);
     count_work(kCtrBeamHit, hits);
     if (overflow) flag_status(kErrTraversalStack);
+}
+
+// The BP2D test of one beam-map leaf against a point: the exact ray-disc
+// predicate on the whole beam; the chunk holding its closest point reports it.
+UPBP_D bool beam_chunk_vs_point(const BeamMap& map, int i, float3 x, float r2, unsigned& beam, float& dist, float& rad2)
+{
+    const uint2 ch = __ldg(&map.chunk[i]);
+    beam = ch.x & 0x7fffffffu;
+    const float4 s0 = __ldg(&map.beams[beam].q[0]), s1 = __ldg(&map.beams[beam].q[1]);
+    if (!pred_ray_disc(xyz(s0), xyz(s1), 0.f, s0.w, x, r2, dist, rad2)) return false;
+    const unsigned k = ch.y & 0xffffu, n = ch.y >> 16;
+    return dist >= chunk_t(s0.w, k, n) && dist < chunk_t(s0.w, k + 1, n);
 }
 
 // Photon beams whose disc of radius sqrt(r2) contains x (BP2D):
@@ -166,13 +171,12 @@ UPBP_D void beams_near_point(const BeamMap& map, float3 x, float r2, F&& f)
     const bool ok = bvh_walk(
         map.bvh, [&](float3 lo, float3 hi) { return inside(lo, hi, x); },
         [&](int i) {
-            const float4 s0 = __ldg(&map.seg[3 * i]), s1 = __ldg(&map.seg[3 * i + 1]);
-            const float4 s2 = __ldg(&map.seg[3 * i + 2]);
             float dist, rad2;
+            unsigned beam;
             cand++;
-            if (pred_ray_disc(xyz(s0), xyz(s1), 0.f, s0.w, x, r2, dist, rad2) && dist >= s2.x && dist < s2.y) {
+            if (beam_chunk_vs_point(map, i, x, r2, beam, dist, rad2)) {
                 hits++;
-                f(fbits(s1.w) & 0x7fffffffu, dist, rad2);
+                f(beam, dist, rad2);
             }
             return true;
         });
