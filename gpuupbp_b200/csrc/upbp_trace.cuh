@@ -31,6 +31,21 @@ struct BoundaryStack {
     Boundary el[kMaxStack];
     int pri[kMaxStack];
 
+    BoundaryStack() = default;
+    UPBP_D BoundaryStack(const BoundaryStack& o) { *this = o; }
+    // Copies the elements in use only: the whole array is 61 words of local
+    // memory, read and written three times per ray, where a path is rarely
+    // inside more than two boundaries.
+    UPBP_D BoundaryStack& operator=(const BoundaryStack& o)
+    {
+        size = o.size;
+#pragma unroll 1
+        for (int i = 0; i < o.size; i++) {
+            el[i] = o.el[i];
+            pri[i] = o.pri[i];
+        }
+        return *this;
+    }
     UPBP_D void clear() { size = 0; }
     UPBP_D bool push(Boundary b, int p)
     {
