@@ -288,7 +288,9 @@ __global__ void k_quantize(const BvhNode* nodes, int n_internal, QNode4* q)
     }
     const int kid[2] = {nodes[i].link.x, nodes[i].link.y};
     for (int s = 1; s >= 0; s--) {
-        if (kid[s] < 0) {
+        // (a clustered tree is quantised before its check is read: a link out
+        // of range, of a tree that will be replaced, is not followed)
+        if (kid[s] < 0 || kid[s] >= n_internal) {
             link[s] = (unsigned)leaf_first(kid[s]) | kQnodeLeaf0 | kQnodeSingle;
             for (int ax = 0; ax < 3; ax++) {  // child 0 of its pair; the other one does not count
                 lo[2 * s][ax] = lo[2 * s + 1][ax] = s ? lo1[ax] : lo[0][ax];
