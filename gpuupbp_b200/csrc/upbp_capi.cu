@@ -267,9 +267,8 @@ struct upbp_ctx {
     bool ploc_pending = false;     // its outcome is not read yet
     BoxSource ploc_src{};          // the build's source and size, to replace the tree
     unsigned ploc_n = 0;
-    int ploc_budget = kPlocPasses;  // passes launched for the next beam map
     int ploc_cap = kPlocPasses;     // UPBP_PLOC_PASSES: at most this many
-    int ploc_failures = 0;          // builds that ran out with every pass allowed
+    int ploc_failures = 0;          // builds that ran out of passes
     bool ploc_off = false;  // UPBP_BEAM_MAP=lbvh: the beam map as a Morton-split LBVH
     void* d_scan_temp = nullptr;
     size_t scan_temp_bytes = 0;
@@ -824,10 +823,8 @@ int alloc_scratch(BuildScratch& sc, unsigned cap)
 
 void free_ploc(PlocScratch& ps)
 {
-    if (ps.exec) cudaGraphExecDestroy(ps.exec);
-    if (ps.capture) cudaStreamDestroy(ps.capture);
-    void* b[] = {ps.cl[0], ps.cl[1], ps.leaf,       ps.nn,      ps.flag,    ps.tile_sum,
-                 ps.node_box, ps.node_child, ps.node_place, ps.written, ps.order, ps.count};
+    void* b[] = {ps.cl[0],    ps.cl[1],      ps.leaf,    ps.act,     ps.block_sum, ps.node_box,
+                 ps.node_child, ps.node_up, ps.written, ps.order, ps.count};
     for (void* x : b)
         if (x) cudaFree(x);
     ps = PlocScratch{};
@@ -838,19 +835,23 @@ void free_ploc(PlocScratch& ps)
 void alloc_ploc(PlocScratch& ps, unsigned cap)
 {
     free_ploc(ps);
-    bool ok = dalloc(&ps.cl[0], 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.cl[1], 2 * (size_t)cap) == cudaSuccess &&
-              dalloc(&ps.leaf, 2 * (size_t)cap) == cudaSuccess &&
-              dalloc(&ps.nn, cap) == cudaSuccess && dalloc(&ps.flag, cap) == cudaSuccess &&
-              dalloc(&ps.tile_sum, cap / kPlocTile + 1) == cudaSuccess &&
-              dalloc(&ps.node_box, 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.node_child, cap) == cudaSuccess &&
-              dalloc(&ps.node_place, cap) == cudaSuccess && dalloc(&ps.written, cap) == cudaSuccess &&
-              dalloc(&ps.order, cap) == cudaSuccess && dalloc(&ps.count, kPcWords) == cudaSuccess;
-    if (ok && cudaStreamCreateWithFlags(&ps.capture, cudaStreamNonBlocking) != cudaSuccess) ps.capture = nullptr;
+    int dev = 0, sms = 0, per_sm = 0;
+    const bool ok =
+        cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ploc_cluster, kPlocBlock, 0) == cudaSuccess &&
+        sms * per_sm > 0 && dalloc(&ps.cl[0], 2 * (size_t)cap) == cudaSuccess &&
+        dalloc(&ps.cl[1], 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.leaf, 2 * (size_t)cap) == cudaSuccess &&
+        dalloc(&ps.act, cap) == cudaSuccess && dalloc(&ps.block_sum, (size_t)sms * per_sm) == cudaSuccess &&
+        dalloc(&ps.node_box, 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.node_child, cap) == cudaSuccess &&
+        dalloc(&ps.node_up, cap) == cudaSuccess && dalloc(&ps.written, cap) == cudaSuccess &&
+        dalloc(&ps.order, cap) == cudaSuccess && dalloc(&ps.count, kPcWords) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_ploc(ps);
         return;
     }
+    ps.grid = sms * per_sm;
     ps.capacity = cap;
 }
 
@@ -1246,7 +1247,6 @@ extern "C" int upbp_create(const upbp_scene_desc* s, const upbp_config* cfg, upb
             const int v = std::atoi(e);
             if (v > 0) c->ploc_cap = std::min(v, kPlocPasses);
         }
-        c->ploc_budget = c->ploc_cap;
         if (const char* e = std::getenv("UPBP_MAX_HITS")) {
             const long long v = std::atoll(e);
             if (v > 0) c->max_hits = std::min<size_t>((size_t)v, kMaxHits);
@@ -1585,11 +1585,8 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 alloc_ploc(c->ploc, nchunks + nchunks / 4);
             }
             if (!c->ploc_off && nchunks >= 2 && nchunks <= c->ploc.capacity) {
-                // the passes the last build needed and a margin: a build that
-                // runs out falls back to the LBVH and the next gets them all
-                const int budget = c->ploc_budget;
                 UPBP_CK(build_ploc(src, nchunks, c->d_beam_nodes, c->sc, c->ploc, c->st, &order, &launches,
-                                   c->h_ploc, budget));
+                                   c->h_ploc, c->ploc_cap));
                 clustered = true;
                 c->ploc_pending = true;  // checked after the camera pass's synchronisation
                 c->ploc_src = src;
@@ -1674,14 +1671,12 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             const unsigned n = c->ploc_n;
             if (ploc_complete(c->h_ploc, n)) {
                 c->beam_map_passes = c->h_ploc[kPcPasses] + c->h_ploc[kPcTailIters];
-                c->ploc_budget = std::min((int)c->h_ploc[kPcPasses] + 4, c->ploc_cap);
             } else {
                 // replaced by the LBVH; a context whose builds run out of
                 // passes even with all of them (boxes too alike to merge
                 // fast) builds the LBVH from then on
                 c->beam_map_passes = 0;
-                if (c->ploc_budget >= c->ploc_cap && ++c->ploc_failures >= 2) c->ploc_off = true;
-                c->ploc_budget = c->ploc_cap;
+                if (++c->ploc_failures >= 2) c->ploc_off = true;
                 const unsigned* order = nullptr;
                 UPBP_CK(build_lbvh(c->ploc_src, n, c->d_beam_nodes, c->sc, c->st, &order));
                 k_gather_chunks<<<(n + 255) / 256, 256, 0, c->st>>>(c->d_chunks, c->d_beams, order, n,
