@@ -281,33 +281,23 @@ UPBP_D void sphere_hit(TriHit& h, float t, float3 n, int k)
     h.prim = ~k;
 }
 
+// Ray casts are made by whole warps (every lane calls; `on` tells which have a
+// ray): the steps of a walk end with a vote, which keeps the lanes together.
+
 // Closest triangle hit with t in [tmin, best] (updates best); ordered
 // traversal, near child first.
-UPBP_D bool closest_triangle(const TriView& tv, float3 o, float3 d, float tmin, float& best, TriHit& hit,
-                             bool& overflow)
+UPBP_D bool closest_triangle(bool on, const TriView& tv, float3 o, float3 d, float tmin, float& best,
+                             TriHit& hit, bool& overflow)
 {
     bool found = false;
     const float3 inv = safe_inv(d);
     int stack[kStackDepth];
     int sp = 0;
-    int node = tv.bvh.count > 1 ? 0 : ~0;
+    int node = on ? (tv.bvh.count > 1 ? 0 : ~0) : kWalkDone;
     unsigned visits = 0, tests = 0;
-    for (;;) {
-        if (node < 0) {
-            const int first = leaf_first(node), cnt = leaf_count(node);
-            for (int s = first; s < first + cnt; s++) {
-                float t, u, v;
-                tests++;
-                if (tri_intersect(tv.tri, s, o, d, t, u, v) && t >= tmin && t <= best) {
-                    best = t;
-                    hit.t = t;
-                    hit.u = u;
-                    hit.v = v;
-                    hit.prim = __float_as_int(__ldg(&tv.tri[3 * s]).w);
-                    found = true;
-                }
-            }
-        } else {
+    while (__any_sync(~0u, node != kWalkDone)) {
+        bool pop = false;
+        if (node >= 0) {
             visits++;
             const NodeBoxes nb = load_node(tv.bvh.nodes, node);
             // entry distances for ordering
@@ -326,22 +316,34 @@ UPBP_D bool closest_triangle(const TriView& tv, float3 o, float3 d, float tmin, 
                     overflow = true;
                 }
                 node = left_first ? nb.l : nb.r;
-                continue;
-            }
-            if (hl) {
-                node = nb.l;
-                continue;
-            }
-            if (hr) {
-                node = nb.r;
-                continue;
+            } else if (hl || hr) {
+                node = hl ? nb.l : nb.r;
+            } else {
+                pop = true;
             }
         }
-        if (sp == 0) break;
-        node = stack[--sp];
+        if (!pop && node < 0 && node != kWalkDone) {
+            const int first = leaf_first(node), cnt = leaf_count(node);
+            for (int s = first; s < first + cnt; s++) {
+                float t, u, v;
+                tests++;
+                if (tri_intersect(tv.tri, s, o, d, t, u, v) && t >= tmin && t <= best) {
+                    best = t;
+                    hit.t = t;
+                    hit.u = u;
+                    hit.v = v;
+                    hit.prim = __float_as_int(__ldg(&tv.tri[3 * s]).w);
+                    found = true;
+                }
+            }
+            pop = true;
+        }
+        if (pop) node = sp > 0 ? stack[--sp] : kWalkDone;
     }
-    count_work(kCtrNodes, visits);
-    count_work(kCtrTris, tests);
+    if (on) {
+        count_work(kCtrNodes, visits);
+        count_work(kCtrTris, tests);
+    }
     return found;
 }
 
@@ -360,11 +362,13 @@ constexpr bool kSceneSpheres = true;
 // (tmin, tmax): a sphere reports its near root when that lies in range, else
 // its far root.  The spheres are tested after the tree, so that nothing of
 // theirs is live during the walk.
-UPBP_D bool closest_hit(const TriView& tv, float3 o, float3 d, float tmin, float tmax, TriHit& hit, bool& overflow)
+UPBP_D bool closest_hit(bool on, const TriView& tv, float3 o, float3 d, float tmin, float tmax, TriHit& hit,
+                        bool& overflow)
 {
     bool found = false;
     float best = tmax;
-    if (tv.bvh.count > 0) found = closest_triangle(tv, o, d, tmin, best, hit, overflow);
+    if (tv.bvh.count > 0) found = closest_triangle(on, tv, o, d, tmin, best, hit, overflow);
+    if (!on) return false;
     for (int k = 0; kSceneSpheres && k < tv.sphere_count; k++) {
         float t1, t2;
         float3 n1, n2;
@@ -384,39 +388,140 @@ UPBP_D bool closest_hit(const TriView& tv, float3 o, float3 d, float tmin, float
     return found;
 }
 
-// Every triangle hit with t in [tmin, tmax], then every sphere root with t in
-// (tmin, tmax) (near root first: the reference's any-hit program ignores
-// each hit, so both roots are reported); calls f(hit) for each, f returns
-// false to stop.
+// The stack of a warp's all_hits: (link, lane that owns the ray) entries.
+constexpr int kAllHitsStack = 448;
+constexpr int kRayWarps = 4;  // warps of the blocks that cast rays
+// Triangles few enough to test one after the other, the lanes together (the
+// boxes of the predefined scenes: camera extend 0.34 -> 0.27 ms at 512x512); a
+// sphere of 1280 triangles is faster shared.
+constexpr unsigned kFewTriangles = 16;
+struct AllHitsStack {
+    int link[kAllHitsStack];
+    unsigned char owner[kAllHitsStack];
+};
+__shared__ AllHitsStack s_all_hits[kRayWarps];
+
+// Every triangle hit with t in [tmin, tmax], in no order but each with its
+// leaf position (h.u, as an int; ascending positions are the order of a
+// left-first walk), then every sphere root with t in (tmin, tmax) (near root
+// first: the reference's any-hit program ignores each hit, so both roots are
+// reported); calls f(hit) on the ray's lane for each, f returns false to stop
+// the ray.
+// The lanes of the warp share the work: 32 (node, ray) entries are tested at
+// once, whichever rays they belong to.  A walk per lane kept 32 lanes waiting
+// for the longest of 32 walks of very different lengths, a memory latency a
+// node (a quarter of the light pass and half of the camera pass; path tracing
+// alone at 960x540, before -> now: light pass 3.34 -> 2.80, camera extend
+// 3.92 -> 3.30 ms).  What bounds the path kernels now: memory latency of the
+// closest-hit walks and of their local arrays, and divergence between bounces.
 template <class F>
-UPBP_D bool all_hits(const TriView& tv, float3 o, float3 d, float tmin, float tmax, F&& f)
+UPBP_D bool all_hits(bool on, const TriView& tv, float3 o, float3 d, float tmin, float tmax, F&& f)
 {
     const float3 inv = safe_inv(d);
-    unsigned tests = 0;
-    bool go = true;
-    count_work(kCtrRays, 1u);
-    const bool ok = bvh_walk(
-        tv.bvh,
-        [&](float3 lo, float3 hi) {
-            const float3 t0 = (lo - o) * inv, t1 = (hi - o) * inv;
-            const float n = fmaxf(fmaxf(fminf(t0.x, t1.x), fminf(t0.y, t1.y)), fmaxf(fminf(t0.z, t1.z), tmin));
-            const float fa = fminf(fminf(fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y)), fminf(fmaxf(t0.z, t1.z), tmax));
-            return n <= fa * 1.00001f + 1e-7f;
-        },
-        [&](int s) {
-            float t, u, v;
-            tests++;
-            if (tri_intersect(tv.tri, s, o, d, t, u, v) && t >= tmin && t <= tmax) {
-                TriHit h;
-                h.t = t;
-                h.u = u;
-                h.v = v;
-                h.prim = __float_as_int(__ldg(&tv.tri[3 * s]).w);
-                go = f(h);
-                return go;
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    AllHitsStack& st = s_all_hits[threadIdx.x >> 5];
+    unsigned visits = 0, tests = 0;
+    bool go = true, ok = true;
+    const bool few = tv.bvh.count <= kFewTriangles;
+    for (int s = 0; few && s < (int)tv.bvh.count; s++) {
+        float t, u, v;
+        if (!on || !go) continue;
+        tests++;
+        if (tri_intersect(tv.tri, s, o, d, t, u, v) && t >= tmin && t <= tmax) {
+            TriHit h;
+            h.t = t;
+            h.u = __int_as_float(s);
+            h.v = 0.f;
+            h.prim = __float_as_int(__ldg(&tv.tri[3 * s]).w);
+            go = f(h);
+        }
+    }
+    const unsigned rays = __ballot_sync(~0u, on && !few);
+    int sp = __popc(rays);
+    if (on && !few) {
+        st.link[__popc(rays & below)] = tv.bvh.count > 1 ? 0 : ~0;
+        st.owner[__popc(rays & below)] = (unsigned char)lane;
+    }
+    while (sp > 0) {
+        __syncwarp();
+        // all lanes while a step leaves room for a depth-first walk, then one entry at a time
+        const int n = max(1, min(min(sp, 32), kAllHitsStack - kStackDepth - sp));
+        const bool mine = (int)lane < n;
+        const int node = mine ? st.link[sp - 1 - lane] : 0;
+        const int owner = mine ? (int)st.owner[sp - 1 - lane] : 0;
+        sp -= n;
+        __syncwarp();
+        const float3 ro = make_float3(__shfl_sync(~0u, o.x, owner), __shfl_sync(~0u, o.y, owner), __shfl_sync(~0u, o.z, owner));
+        const float t0r = __shfl_sync(~0u, tmin, owner), t1r = __shfl_sync(~0u, tmax, owner);
+        const float3 ri = make_float3(__shfl_sync(~0u, inv.x, owner), __shfl_sync(~0u, inv.y, owner), __shfl_sync(~0u, inv.z, owner));
+        const float3 rd = make_float3(__shfl_sync(~0u, d.x, owner), __shfl_sync(~0u, d.y, owner), __shfl_sync(~0u, d.z, owner));
+        const bool live = __shfl_sync(~0u, (int)go, owner) != 0;
+        bool hl = false, hr = false;
+        int cl = 0, cr = 0;
+        if (mine && live && node >= 0) {
+            visits++;
+            const NodeBoxes nb = load_node(tv.bvh.nodes, node);
+            auto test = [&](float3 lo, float3 hi) {
+                const float3 t0 = (lo - ro) * ri, t1 = (hi - ro) * ri;
+                const float n = fmaxf(fmaxf(fminf(t0.x, t1.x), fminf(t0.y, t1.y)), fmaxf(fminf(t0.z, t1.z), t0r));
+                const float fa = fminf(fminf(fmaxf(t0.x, t1.x), fmaxf(t0.y, t1.y)), fminf(fmaxf(t0.z, t1.z), t1r));
+                return n <= fa * 1.00001f + 1e-7f;
+            };
+            hl = test(nb.llo, nb.lhi);
+            hr = test(nb.rlo, nb.rhi);
+            cl = nb.l;
+            cr = nb.r;
+        }
+        const unsigned ml = __ballot_sync(~0u, hl), mr = __ballot_sync(~0u, hr);
+        int at = sp + __popc(ml & below) + __popc(mr & below);
+        if (hl) {
+            if (at < kAllHitsStack) {
+                st.link[at] = cl;
+                st.owner[at] = (unsigned char)owner;
             }
-            return true;
-        });
+            at++;
+        }
+        if (hr && at < kAllHitsStack) {
+            st.link[at] = cr;
+            st.owner[at] = (unsigned char)owner;
+        }
+        sp += __popc(ml) + __popc(mr);
+        if (sp > kAllHitsStack) {
+            sp = kAllHitsStack;
+            ok = false;
+        }
+        // leaves: each hit goes to the ray's lane
+        const bool leaf = mine && live && node < 0;
+        if (!__any_sync(~0u, leaf)) continue;
+        const int first = leaf ? leaf_first(node) : 0, cnt = leaf ? leaf_count(node) : 0;
+        for (int k = 0; __any_sync(~0u, k < cnt); k++) {
+            float t = 0.f, u, v;
+            bool hit = false;
+            if (k < cnt) {
+                tests++;
+                hit = tri_intersect(tv.tri, first + k, ro, rd, t, u, v) && t >= t0r && t <= t1r;
+            }
+            for (unsigned m = __ballot_sync(~0u, hit); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const int to = __shfl_sync(~0u, owner, src), s = __shfl_sync(~0u, first + k, src);
+                const float ht = __shfl_sync(~0u, t, src);
+                if ((int)lane == to && go) {
+                    TriHit h;
+                    h.t = ht;
+                    h.u = __int_as_float(s);
+                    h.v = 0.f;
+                    h.prim = __float_as_int(__ldg(&tv.tri[3 * s]).w);
+                    go = f(h);
+                }
+            }
+        }
+    }
+    count_work(kCtrNodes, visits);
+    if (!on) {
+        count_work(kCtrTris, tests);
+        return ok;
+    }
+    count_work(kCtrRays, 1u);
     for (int k = 0; kSceneSpheres && k < tv.sphere_count && go; k++) {
         float t1, t2;
         float3 n1, n2;

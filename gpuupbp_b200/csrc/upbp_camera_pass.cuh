@@ -112,7 +112,7 @@ UPBP_D bool nee_sample(NeeSample& ns, float3 hit, const Bsdf& bsdf, Rng& rng)
     return true;
 }
 
-UPBP_D unsigned nee_finish(float3& contrib, const NeeSample& ns, float3 hit, bool in_medium, const BoundaryStack& stack,
+UPBP_D unsigned nee_finish(bool on, float3& contrib, const NeeSample& ns, float3 hit, bool in_medium, const BoundaryStack& stack,
                            const VertexWeights& wc, VolSeg* segs, float* w_out = nullptr, int* nseg_out = nullptr)
 {
     contrib = v3(0.f);
@@ -120,7 +120,9 @@ UPBP_D unsigned nee_finish(float3& contrib, const NeeSample& ns, float3 hit, boo
     bool occ;
     Rng unused;
     unused.state = unused.inc = 0;  // occlusion rays draw no random numbers
-    const unsigned st = occluded(occ, hit, ns.dir, ns.dist, stack, in_medium ? kOriginInMedium : 0u, segs, nseg, unused);
+    const unsigned st =
+        occluded(on, occ, hit, ns.dir, ns.dist, stack, in_medium ? kOriginInMedium : 0u, segs, nseg, unused);
+    if (!on) return 0;
     if (st) return st;
     if (occ) return 0;
     float n_rev = 1.f, n_for = 1.f;
@@ -147,35 +149,46 @@ UPBP_D unsigned nee_finish(float3& contrib, const NeeSample& ns, float3 hit, boo
 }
 
 // BPT connection of a camera and a light vertex, Eq 4.50/4.51
-// (functs_camera.cuh:349-527).
-UPBP_D unsigned connect_vertices(float3& contrib, const LightVertex& lv, const Bsdf& cb, float3 chit, const PathState& s,
+// (functs_camera.cuh:349-527).  The whole warp calls it; `on` tells which
+// lanes have a pair.
+UPBP_D unsigned connect_vertices(bool on, float3& contrib, const LightVertex& lv, const Bsdf& cb, float3 chit, const PathState& s,
                                  Rng& rng, VolSeg* segs, float* w_out = nullptr, int* nseg_out = nullptr)
 {
     contrib = v3(0.f);
-    float3 dir = lv.hit - chit;
-    const float d2 = dot(dir, dir);
-    const float dist = sqrtf(d2);
-    dir /= dist;
-    float cos_c, c_fpdf, c_rpdf, sin_c;
-    const float3 cf = bsdf_eval(cb, dir, cos_c, &c_fpdf, &c_rpdf, &sin_c);
-    if (is_black_or_negative(cf)) return 0;
-    c_fpdf *= cb.cont_prob;
-    c_rpdf *= cb.cont_prob;
-    float cos_l, l_fpdf, l_rpdf, sin_l;
-    const float3 lf = bsdf_eval(lv.bsdf, -dir, cos_l, &l_fpdf, &l_rpdf, &sin_l);
-    if (is_black_or_negative(lf)) return 0;
-    l_fpdf *= lv.bsdf.cont_prob;
-    l_rpdf *= lv.bsdf.cont_prob;
-    const float g = cos_l * cos_c / d2;
-    if (g < 0.f) return 0;
-    const float c_fpdf_a = pdf_w_to_a(c_fpdf, dist, cos_l);
-    const float l_fpdf_a = pdf_w_to_a(l_fpdf, dist, cos_c);
+    float3 dir = v3(0.f), cf = v3(0.f), lf = v3(0.f);
+    float dist = 0.f, sin_c = 0.f, c_rpdf = 0.f, sin_l = 0.f, l_rpdf = 0.f, g = 0.f, c_fpdf_a = 0.f, l_fpdf_a = 0.f;
+    bool cast = false;
+    do {
+        if (!on) break;
+        dir = lv.hit - chit;
+        // the multiply-adds written out: the last bit of the distance decides
+        // some occlusion tests, and the compiler's choice depends on the code around
+        const float d2 = fmaf(dir.z, dir.z, fmaf(dir.x, dir.x, dir.y * dir.y));
+        dist = sqrtf(d2);
+        dir /= dist;
+        float cos_c, c_fpdf;
+        cf = bsdf_eval(cb, dir, cos_c, &c_fpdf, &c_rpdf, &sin_c);
+        if (is_black_or_negative(cf)) break;
+        c_fpdf *= cb.cont_prob;
+        c_rpdf *= cb.cont_prob;
+        float cos_l, l_fpdf;
+        lf = bsdf_eval(lv.bsdf, -dir, cos_l, &l_fpdf, &l_rpdf, &sin_l);
+        if (is_black_or_negative(lf)) break;
+        l_fpdf *= lv.bsdf.cont_prob;
+        l_rpdf *= lv.bsdf.cont_prob;
+        g = cos_l * cos_c / d2;
+        if (g < 0.f) break;
+        c_fpdf_a = pdf_w_to_a(c_fpdf, dist, cos_l);
+        l_fpdf_a = pdf_w_to_a(l_fpdf, dist, cos_c);
+        cast = true;
+    } while (false);
     unsigned sflags = 0;
-    if (cb.in_medium()) sflags |= kOriginInMedium;
-    if (lv.in_medium) sflags |= kEndInMedium;
+    if (cast && cb.in_medium()) sflags |= kOriginInMedium;
+    if (cast && lv.in_medium) sflags |= kEndInMedium;
     int nseg = 0;
     bool occ;
-    const unsigned st = occluded(occ, chit, dir, dist, s.stack, sflags, segs, nseg, rng);
+    const unsigned st = occluded(cast, occ, chit, dir, dist, s.stack, sflags, segs, nseg, rng);
+    if (!cast) return 0;
     if (st) return st;
     if (occ) return 0;
     float rs_for = 1.f, rs_rev = 1.f;
@@ -864,8 +877,9 @@ UPBP_D bool camera_path_begin(CameraLane& c, unsigned pixel)
 }
 
 // One bounce of a camera subpath (one iteration of the path loop of
-// __raygen__trace_camera, trace_camera.cu:79-381); false when the path ends.
-UPBP_D bool camera_path_bounce(CameraLane& c, VolSeg* segs, LiteSeg* lsegs)
+// __raygen__trace_camera, trace_camera.cu:79-381), by whole warps (`on`
+// tells which lanes have a path); false when the path ends.
+UPBP_D bool camera_path_bounce(bool on, CameraLane& c, VolSeg* segs, LiteSeg* lsegs)
 {
     const DeviceParams& p = c_params;
     PathState& s = c.s;
@@ -883,8 +897,10 @@ UPBP_D bool camera_path_bounce(CameraLane& c, VolSeg* segs, LiteSeg* lsegs)
     isect.enter = false;
     int nseg = 0, nlseg = 0;
     bool hit;
-    ret = intersect_scene(hit, ro, rd, isect, s.stack, kSampleScattering, origin_in_medium ? kOriginInMedium : 0u,
-                          segs, nseg, lsegs, nlseg, rng);
+    const unsigned st = intersect_scene(on, hit, ro, rd, isect, s.stack, kSampleScattering,
+                                        origin_in_medium ? kOriginInMedium : 0u, segs, nseg, lsegs, nlseg, rng);
+    if (!on) return false;
+    ret = st;
     if (ret) return false;
     UPBP_MISDBG(mis_ray(false, c.path, s.path_length, rd, hit ? isect.dist : kInfinity,
                         origin_in_medium ? kOriginInMedium : 0u, lsegs, nlseg));
@@ -1077,8 +1093,12 @@ __global__ void __launch_bounds__(128, 8) camera_pass_kernel(int slot)
                 }
             }
         }
-        if (__all_sync(~0u, exhausted && !active)) break;
-        if (active && !camera_path_bounce(c, segs, lsegs)) {
+        if (!__any_sync(~0u, active)) {
+            if (__all_sync(~0u, exhausted)) break;
+            continue;
+        }
+        const bool goes_on = camera_path_bounce(active, c, segs, lsegs);
+        if (active && !goes_on) {
             camera_path_end(c);
             active = false;
         }
@@ -1095,8 +1115,9 @@ __global__ void __launch_bounds__(128, 8) nee_connect_kernel(int slot)
     const unsigned n = min(p.queue_count[4], p.nee_capacity);
     VolSeg segs[kMaxVolSegments];
     BoundaryStack st;
-    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const float4* q = p.nee_queue[j].q;
+    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; __any_sync(~0u, j < n); j += gridDim.x * blockDim.x) {
+        const bool on = j < n;
+        const float4* q = p.nee_queue[on ? j : 0u].q;  // (lanes past the end only help with the rays)
         const float4 q0 = __ldg(&q[0]), q1 = __ldg(&q[1]), q2 = __ldg(&q[2]), q3 = __ldg(&q[3]), q4 = __ldg(&q[4]);
         NeeSample ns;
         const float3 hit = xyz(q0);
@@ -1127,7 +1148,8 @@ __global__ void __launch_bounds__(128, 8) nee_connect_kernel(int slot)
         float3 c;
         float w = -1.f;
         int nseg = 0;
-        const unsigned e = nee_finish(c, ns, hit, in_medium, st, wc, segs, &w, &nseg);
+        const unsigned e = nee_finish(on, c, ns, hit, in_medium, st, wc, segs, &w, &nseg);
+        if (!on) continue;
         UPBP_MISDBG(if (!e && w >= 0.f) {
             MisEvent ev{kMisNee, fbits(q8.z), fbits(q8.w), 0u, 0u, fbits(q4.w) >> 1, w, hit + ns.dir * ns.dist, hit,
                         0.f, 0.f};
@@ -1155,28 +1177,37 @@ __global__ void __launch_bounds__(128, 8) bpt_connect_kernel(int slot)
     VolSeg segs[kMaxVolSegments];
     PathState ps;
     unsigned loads = 0;
-    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const uint2 pr = __ldg(&p.bpt_pairs[j]);
-        const ConnVertexRec* cr = p.conn_vertices + pr.x;
-        p.bpt_color[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; __any_sync(~0u, j < n); j += gridDim.x * blockDim.x) {
+        bool on = j < n;
+        uint2 pr = make_uint2(0u, 0u);
+        const ConnVertexRec* cr = p.conn_vertices;
         LightVertex lv, cv;
-        load_vertex(p.vertices + pr.y, lv);
-        loads++;
-        load_vertex(&cr->v, cv);
-        const unsigned plen = lv.path_length + 1 + cv.path_length;
-        if (plen > p.max_path_length || plen < p.min_path_length) continue;
-        const bool diff_media = lv.bsdf.in_medium() && cv.bsdf.in_medium() && lv.bsdf.id != cv.bsdf.id &&
-                                (lv.behind_surf || cv.behind_surf);
-        if (diff_media) continue;
-        const float4 q8 = __ldg(&cr->q8);
-        load_conn_stack(cr, fbits(q8.y), ps.stack);
-        ps.sw.w = cv.w;
+        float4 q8 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on) {
+            pr = __ldg(&p.bpt_pairs[j]);
+            cr = p.conn_vertices + pr.x;
+            p.bpt_color[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            load_vertex(p.vertices + pr.y, lv);
+            loads++;
+            load_vertex(&cr->v, cv);
+            const unsigned plen = lv.path_length + 1 + cv.path_length;
+            if (plen > p.max_path_length || plen < p.min_path_length) on = false;
+            const bool diff_media = lv.bsdf.in_medium() && cv.bsdf.in_medium() && lv.bsdf.id != cv.bsdf.id &&
+                                    (lv.behind_surf || cv.behind_surf);
+            if (diff_media) on = false;
+            if (on) {
+                q8 = __ldg(&cr->q8);
+                load_conn_stack(cr, fbits(q8.y), ps.stack);
+                ps.sw.w = cv.w;
+            }
+        }
         Rng unused;
         unused.state = unused.inc = 0;  // occlusion rays draw no random numbers
         float3 c;
         float w = -1.f;
         int nseg = 0;
-        const unsigned e = connect_vertices(c, lv, cv.bsdf, cv.hit, ps, unused, segs, &w, &nseg);
+        const unsigned e = connect_vertices(on, c, lv, cv.bsdf, cv.hit, ps, unused, segs, &w, &nseg);
+        if (!on) continue;
         UPBP_MISDBG(if (!e && w >= 0.f) {
             MisEvent ev{kMisBpt, fbits(q8.z), fbits(q8.w), pr.y / p.slots_per_path, lv.path_length, 0u, w, lv.hit,
                         cv.hit, 0.f, 0.f};

@@ -94,30 +94,41 @@ UPBP_D void add_beams(float3 ro, float3 rd, float3 throughput, unsigned path_len
 }
 
 // Light tracing splat to the image plane (functs_light.cuh:251-388, Eq D.38).
-UPBP_D unsigned connect_to_camera(const PathState& s, float3 hit, const Bsdf& bsdf, Rng& rng, VolSeg* segs,
+// The whole warp calls it; `on` tells which lanes connect a vertex.
+UPBP_D unsigned connect_to_camera(bool on, const PathState& s, float3 hit, const Bsdf& bsdf, Rng& rng, VolSeg* segs,
                                   unsigned path_idx)
 {
     const DeviceParams& p = c_params;
     const DCamera& cam = p.camera;
-    float3 to_cam = cam.origin - hit;
-    if (dot(cam.direction, -to_cam) <= 0.f) return 0;
-    const float2 ip = world_to_raster(cam, hit);
-    if (!raster_inside(cam, ip)) return 0;
-    const float d2 = dot(to_cam, to_cam);
-    const float dist = sqrtf(d2);
-    to_cam /= dist;
-    float cos_to_cam, fpdf, rpdf, sin_theta;
-    const float3 f = bsdf_eval(bsdf, to_cam, cos_to_cam, &fpdf, &rpdf, &sin_theta);
-    if (is_black_or_negative(f)) return 0;
-    rpdf *= bsdf.cont_prob;
-    const float cos_at_cam = dot(cam.direction, -to_cam);
-    const float ip_dist = cam.image_plane_dist / cos_at_cam;
-    const float i2sa = ip_dist * ip_dist / cos_at_cam;
-    const float i2s = i2sa * fabsf(cos_to_cam) / (dist * dist);
+    float3 to_cam = v3(0.f), f = v3(0.f);
+    float2 ip = make_float2(0.f, 0.f);
+    float dist = 0.f, rpdf = 0.f, sin_theta = 0.f, i2s = 0.f;
+    bool cast = false;
+    do {
+        if (!on) break;
+        to_cam = cam.origin - hit;
+        if (dot(cam.direction, -to_cam) <= 0.f) break;
+        ip = world_to_raster(cam, hit);
+        if (!raster_inside(cam, ip)) break;
+        const float d2 = dot(to_cam, to_cam);
+        dist = sqrtf(d2);
+        to_cam /= dist;
+        float cos_to_cam, fpdf;
+        f = bsdf_eval(bsdf, to_cam, cos_to_cam, &fpdf, &rpdf, &sin_theta);
+        if (is_black_or_negative(f)) break;
+        rpdf *= bsdf.cont_prob;
+        const float cos_at_cam = dot(cam.direction, -to_cam);
+        const float ip_dist = cam.image_plane_dist / cos_at_cam;
+        const float i2sa = ip_dist * ip_dist / cos_at_cam;
+        i2s = i2sa * fabsf(cos_to_cam) / (dist * dist);
+        cast = true;
+    } while (false);
     const float camera_pdf_a = i2s;
     int nseg = 0;
     bool occ;
-    const unsigned st = occluded(occ, hit, to_cam, dist, s.stack, bsdf.in_medium() ? kOriginInMedium : 0u, segs, nseg, rng);
+    const unsigned st =
+        occluded(cast, occ, hit, to_cam, dist, s.stack, cast && bsdf.in_medium() ? kOriginInMedium : 0u, segs, nseg, rng);
+    if (!cast) return 0;
     if (st) return st;
     if (occ) return 0;
     float rs_rev = 1.f;
@@ -184,8 +195,11 @@ UPBP_D bool light_path_begin(LightLane& l, unsigned path_idx)
 }
 
 // One bounce of a light subpath (one iteration of the path loop of
-// __raygen__trace_light, trace_light.cu:84-320); false when the path ends.
-UPBP_D bool light_path_bounce(LightLane& l, VolSeg* segs, LiteSeg* lsegs)
+// __raygen__trace_light, trace_light.cu:84-320) up to its connection to the
+// camera, by whole warps (`on` tells which lanes have a path); false when the
+// path ends.
+UPBP_D bool light_path_trace(bool on, LightLane& l, Isect& isect, Bsdf& bsdf, float3& hitpoint, bool& connect,
+                             VolSeg* segs, LiteSeg* lsegs)
 {
     const DeviceParams& p = c_params;
     PathState& s = l.s;
@@ -197,15 +211,16 @@ UPBP_D bool light_path_bounce(LightLane& l, VolSeg* segs, LiteSeg* lsegs)
     bool& origin_in_medium = l.origin_in_medium;
     unsigned& ret = l.ret;
     const float3 ro = s.origin, rd = s.dir;
-    Isect isect;
     isect.dist = kInfinity;
     isect.mat = isect.med = isect.light = -1;
     isect.normal = v3(0.f);
     isect.enter = false;
     int nseg = 0, nlseg = 0;
     bool hit;
-    ret = intersect_scene(hit, ro, rd, isect, s.stack, kSampleScattering, origin_in_medium ? kOriginInMedium : 0u,
-                          segs, nseg, lsegs, nlseg, rng);
+    const unsigned st = intersect_scene(on, hit, ro, rd, isect, s.stack, kSampleScattering,
+                                        origin_in_medium ? kOriginInMedium : 0u, segs, nseg, lsegs, nlseg, rng);
+    if (!on) return false;
+    ret = st;
     if (ret) return false;
     UPBP_MISDBG(mis_ray(true, path_idx, s.path_length, rd, hit ? isect.dist : kInfinity,
                         origin_in_medium ? kOriginInMedium : 0u, lsegs, nlseg));
@@ -233,7 +248,6 @@ UPBP_D bool light_path_bounce(LightLane& l, VolSeg* segs, LiteSeg* lsegs)
     w.d_bpt /= rs_for;
     w.d_pde /= rs_for;
 
-    Bsdf bsdf;
     float3 frame_src;
     if (isect.on_surface()) {
         frame_src = isect.shading_normal;
@@ -245,7 +259,7 @@ UPBP_D bool light_path_bounce(LightLane& l, VolSeg* segs, LiteSeg* lsegs)
     if (!bsdf.valid()) return false;
     float ratio = 0.f;
     if (bsdf.in_medium()) ratio = 1.f / p.media[bsdf.id].min_pos_att;
-    const float3 hitpoint = ro + rd * isect.dist;
+    hitpoint = ro + rd * isect.dist;
     origin_in_medium = isect.in_medium();
     UPBP_MISDBG(mis_hit(true, path_idx, s.path_length, hitpoint, isect.in_medium(),
                         isect.in_medium() ? isect.med : isect.mat, isect.in_medium() ? v3(0.f) : isect.shading_normal,
@@ -290,17 +304,22 @@ UPBP_D bool light_path_bounce(LightLane& l, VolSeg* segs, LiteSeg* lsegs)
             p.guide_recs[k] = GuideRecord{make_float4(hitpoint.x, hitpoint.y, hitpoint.z, ubits((unsigned)bsdf.id)),
                                           make_float4(rd.x, rd.y, rd.z, luminance(s.throughput))};
     }
-    if (p.do_bpt && !bsdf.delta() && (bsdf.in_medium() || p.connect_to_camera_from_surf)) {
-        if (s.path_length + 1 >= p.min_path_length) {
-            ret = connect_to_camera(s, hitpoint, bsdf, rng, segs, path_idx);
-            if (ret) return false;
-        }
-    }
+    connect = p.do_bpt && !bsdf.delta() && (bsdf.in_medium() || p.connect_to_camera_from_surf) &&
+              s.path_length + 1 >= p.min_path_length;
+    return true;
+}
+
+// The rest of the bounce: the next direction; false when the path ends.
+UPBP_D bool light_path_scatter(LightLane& l, const Isect& isect, const Bsdf& bsdf, float3 hitpoint)
+{
+    const DeviceParams& p = c_params;
+    PathState& s = l.s;
+    unsigned& ret = l.ret;
     if (s.path_length + 2 > p.max_path_length) return false;
     bool cont;
-    ret = sample_scattering(cont, bsdf, hitpoint, isect, s, rng);
+    ret = sample_scattering(cont, bsdf, hitpoint, isect, s, l.rng);
     if (ret || !cont) return false;
-    UPBP_MISDBG(if (s.sw.w.prev_specular) mis_specular(true, path_idx, s.path_length));
+    UPBP_MISDBG(if (s.sw.w.prev_specular) mis_specular(true, l.path_idx, s.path_length));
     s.path_length++;
     return true;
 }
@@ -343,8 +362,22 @@ __global__ void __launch_bounds__(128, 8) light_pass_kernel(int slot)
                 }
             }
         }
-        if (__all_sync(~0u, exhausted && !active)) break;
-        if (active && !light_path_bounce(l, segs, lsegs)) {
+        if (!__any_sync(~0u, active)) {
+            if (__all_sync(~0u, exhausted)) break;
+            continue;
+        }
+        // a bounce in three steps, the lanes brought together for each ray
+        Isect isect;
+        Bsdf bsdf;
+        float3 hitpoint = v3(0.f);
+        bool connect = false;
+        bool goes_on = light_path_trace(active, l, isect, bsdf, hitpoint, connect, segs, lsegs);
+        const unsigned ret = connect_to_camera(goes_on && connect, l.s, hitpoint, bsdf, l.rng, segs, l.path_idx);
+        if (goes_on && connect) {
+            l.ret = ret;
+            goes_on = ret == 0;
+        }
+        if (active && !(goes_on && light_path_scatter(l, isect, bsdf, hitpoint))) {
             light_path_end(l);
             active = false;
         }

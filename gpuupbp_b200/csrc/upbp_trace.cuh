@@ -189,10 +189,11 @@ UPBP_D bool init_boundary_stack(BoundaryStack& s)
 // a medium scattering point was found (result.dist), `segs` holds the medium
 // segments up to that point (with sampling pdfs) and `lsegs` the segments up
 // to the next real surface.  Returns a status bit (0 on success).
+// The whole warp calls it; `on` tells which lanes have a ray (upbp_bvh.cuh).
 // Kept out of line: inlined into every caller it made the path kernels too large
 // for the instruction cache.
-__device__ __noinline__ unsigned intersect_scene(bool& hit, float3 ro, float3 rd, Isect& result, BoundaryStack& bstack,
-                                unsigned options, unsigned sflags, VolSeg* segs, int& nseg, LiteSeg* lsegs,
+__device__ __noinline__ unsigned intersect_scene(bool on, bool& hit, float3 ro, float3 rd, Isect& result,
+                                BoundaryStack& bstack, unsigned options, unsigned sflags, VolSeg* segs, int& nseg, LiteSeg* lsegs,
                                 int& nlseg, Rng& rng)
 {
     hit = false;
@@ -204,7 +205,7 @@ __device__ __noinline__ unsigned intersect_scene(bool& hit, float3 ro, float3 rd
 
     LiteHit real_hits[kMaxRealHits];
     int n_real = 0;
-    const int top_priority = bstack.top_priority();
+    const int top_priority = on ? bstack.top_priority() : 0;
     const float first_eps = (sflags & kOriginInMedium) ? 0.f : kEpsRay;
     float t_max, miss_dist;
     if (occlusion) {
@@ -215,40 +216,52 @@ __device__ __noinline__ unsigned intersect_scene(bool& hit, float3 ro, float3 rd
         miss_dist = kInfinity;
     }
 
-    BoundaryStack scopy = bstack;
+    BoundaryStack scopy;
+    if (on) scopy = bstack;
     float t_min = first_eps;
-    bool not_yet_real;
-    do {
-        not_yet_real = false;
-        tmp.dist = kInfinity;
+    bool not_yet_real = false;
+    unsigned err = 0;
+    bool cast = on;  // a real surface is still looked for
+    while (__any_sync(~0u, cast)) {
         TriHit th;
         bool ovf = false;
-        if (closest_hit(c_params.real, ro, rd, t_min, t_max, th, ovf)) fill_hit(c_params.real, th, rd, tmp);
-        if (ovf) flag_status(kErrTraversalStack);
-        hit = tmp.dist != kInfinity;
-        if (hit) {
-            dist = tmp.dist;
-            const int priority = boundary_priority(tmp.mat);
-            const Boundary top = scopy.top();
-            if (tmp.med < 0) tmp.med = top.med;
-            if (priority < top_priority && priority != kThinWallPriority) {
-                const Boundary e{tmp.mat, tmp.med};
-                if (tmp.enter) {
-                    if (n_real == kMaxRealHits) return kErrIntersectionArray;
-                    real_hits[n_real++] = LiteHit{tmp.dist, tmp.mat, tmp.med, 1};
-                    if (!scopy.push(e, priority)) return kErrBoundaryStack;
-                } else if (scopy.pop(e, priority)) {
-                    if (n_real == kMaxRealHits) return kErrIntersectionArray;
-                    real_hits[n_real++] = LiteHit{tmp.dist, tmp.mat, tmp.med, 0};
+        const bool found = closest_hit(cast, c_params.real, ro, rd, t_min, t_max, th, ovf);
+        if (cast) {
+            not_yet_real = false;
+            tmp.dist = kInfinity;
+            if (found) fill_hit(c_params.real, th, rd, tmp);
+            if (ovf) flag_status(kErrTraversalStack);
+            hit = tmp.dist != kInfinity;
+            if (hit) {
+                dist = tmp.dist;
+                const int priority = boundary_priority(tmp.mat);
+                const Boundary top = scopy.top();
+                if (tmp.med < 0) tmp.med = top.med;
+                if (priority < top_priority && priority != kThinWallPriority) {
+                    const Boundary e{tmp.mat, tmp.med};
+                    if (tmp.enter) {
+                        if (n_real == kMaxRealHits) {
+                            err = kErrIntersectionArray;
+                        } else {
+                            real_hits[n_real++] = LiteHit{tmp.dist, tmp.mat, tmp.med, 1};
+                            if (!scopy.push(e, priority)) err = kErrBoundaryStack;
+                        }
+                    } else if (scopy.pop(e, priority)) {
+                        if (n_real == kMaxRealHits)
+                            err = kErrIntersectionArray;
+                        else
+                            real_hits[n_real++] = LiteHit{tmp.dist, tmp.mat, tmp.med, 0};
+                    }
+                    not_yet_real = true;
+                    t_min = dist + kEpsRay;
+                    // the reference shrinks an occlusion query by the skipped distance
+                    // twice (intersector.cuh:167-170); kept for parity
+                    t_max = occlusion ? miss_dist - dist - kEpsRay : kInfinity;
                 }
-                not_yet_real = true;
-                t_min = dist + kEpsRay;
-                // the reference shrinks an occlusion query by the skipped distance
-                // twice (intersector.cuh:167-170); kept for parity
-                t_max = occlusion ? miss_dist - dist - kEpsRay : kInfinity;
             }
+            cast = !err && not_yet_real && t_max > t_min;
         }
-    } while (not_yet_real && t_max > t_min);
+    }
 
     if (!hit || not_yet_real) {
         hit = false;
@@ -260,30 +273,35 @@ __device__ __noinline__ unsigned intersect_scene(bool& hit, float3 ro, float3 rd
     // imaginary boundaries before the real hit
     bool scattered = false;
     LiteHit imag[kMaxImagHits];
-    int n_imag = -1;
-    if (!is_real_material(bstack.top().mat) && dist > first_eps + kEpsRay) {
-        n_imag = 0;
-        bool overflow = false;
-        const bool ok = all_hits(c_params.imag, ro, rd, first_eps, dist - kEpsRay, [&](const TriHit& h) {
-            Isect ih;
-            fill_hit(c_params.imag, h, rd, ih);
-            if (n_imag == kMaxImagHits) {
-                overflow = true;
-                return false;
-            }
-            // sorted insert by distance, after equal distances
-            int i = n_imag - 1;
-            while (i >= 0 && imag[i].dist > ih.dist) {
-                imag[i + 1] = imag[i];
-                i--;
-            }
-            imag[i + 1] = LiteHit{ih.dist, ih.mat, ih.med, ih.enter ? 1 : 0};
-            n_imag++;
-            return true;
-        });
-        if (!ok) flag_status(kErrTraversalStack);
-        if (overflow) return kErrIntersectionStack;
-
+    int imag_pos[kMaxImagHits];  // leaf positions
+    const bool media = on && !err && !is_real_material(bstack.top().mat) && dist > first_eps + kEpsRay;
+    int n_imag = media ? 0 : -1;
+    bool overflow = false;
+    const bool ok = all_hits(media, c_params.imag, ro, rd, first_eps, dist - kEpsRay, [&](const TriHit& h) {
+        Isect ih;
+        fill_hit(c_params.imag, h, rd, ih);
+        if (n_imag == kMaxImagHits) {
+            overflow = true;
+            return false;
+        }
+        // sorted insert by distance; triangles at equal distances in leaf
+        // order (spheres come after the triangles, each after its equals)
+        int i = n_imag - 1;
+        const int pos = h.prim < 0 ? INT_MAX : __float_as_int(h.u);
+        while (i >= 0 && (imag[i].dist > ih.dist || (imag[i].dist == ih.dist && imag_pos[i] > pos))) {
+            imag[i + 1] = imag[i];
+            imag_pos[i + 1] = imag_pos[i];
+            i--;
+        }
+        imag[i + 1] = LiteHit{ih.dist, ih.mat, ih.med, ih.enter ? 1 : 0};
+        imag_pos[i + 1] = pos;
+        n_imag++;
+        return true;
+    });
+    if (!ok) flag_status(kErrTraversalStack);
+    if (!on || err) return err;
+    if (overflow) return kErrIntersectionStack;
+    if (media) {
         scopy = bstack;
         float dmin = 0.f;
         for (int i = 0; i < n_imag; i++) {
@@ -381,11 +399,13 @@ __device__ __noinline__ unsigned intersect_scene(bool& hit, float3 ro, float3 rd
     return 0;
 }
 
-// Occlusion query from `p` toward `dir` up to t_max (intersector.cuh:375-397).
-UPBP_D unsigned occluded(bool& hit, float3 p, float3 dir, float t_max, const BoundaryStack& bstack, unsigned sflags,
+// Occlusion query from `p` toward `dir` up to t_max (intersector.cuh:375-397),
+// by whole warps.
+UPBP_D unsigned occluded(bool on, bool& hit, float3 p, float3 dir, float t_max, const BoundaryStack& bstack, unsigned sflags,
                          VolSeg* segs, int& nseg, Rng& rng)
 {
-    BoundaryStack scopy = bstack;
+    BoundaryStack scopy;
+    if (on) scopy = bstack;
     Isect tmp;
     tmp.dist = t_max;
     tmp.mat = tmp.med = tmp.light = -1;
@@ -394,7 +414,7 @@ UPBP_D unsigned occluded(bool& hit, float3 p, float3 dir, float t_max, const Bou
     LiteSeg lsegs[kMaxVolSegments];
     int nl = 0;
     nseg = 0;
-    return intersect_scene(hit, p, dir, tmp, scopy, kOcclusionTest, sflags, segs, nseg, lsegs, nl, rng);
+    return intersect_scene(on, hit, p, dir, tmp, scopy, kOcclusionTest, sflags, segs, nseg, lsegs, nl, rng);
 }
 
 UPBP_D float relative_ior(const Isect& is, const BoundaryStack& st)
