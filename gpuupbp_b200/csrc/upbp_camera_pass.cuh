@@ -331,8 +331,12 @@ UPBP_D float3 eval_bb1d(const QuerySeg& q, const StateWeights& cw, const Beam& l
     float rsr_p = (lb.flags & kOriginInMedium) ? rsf_p : pp;
     const float3 att = att_c * att_p;
     if (!is_positive(att)) return v3(0.f);
+    // Half of the evaluation's divisions repeated a divisor or inverted an
+    // inverse (an IEEE division is about nine instructions): one reciprocal a
+    // sampling pdf, and the pdf itself where its reciprocal divided.
     rsf_c *= q.for_pdf;
     rsr_c *= q.rev_pdf;
+    const float irf_c = 1.f / rsf_c;
     VertexWeights wc = cw.w;
     if (q.cam_path_length > 1u) {
         const float f_i = pde_factor(wc.prev_in_medium, wc.prev_specular, 1.f / rsr_c, wc.rev_ratio, wc.for_inv,
@@ -342,6 +346,7 @@ UPBP_D float3 eval_bb1d(const QuerySeg& q, const StateWeights& cw, const Beam& l
     }
     rsf_p *= lb.for_pdf;
     rsr_p *= lb.rev_pdf;
+    const float irf_p = 1.f / rsf_p;
     VertexWeights wl = lb.sw.w;
     if (lb.path_length > 1u) {
         const float f_i = pde_factor(wl.prev_in_medium, wl.prev_specular, wl.for_inv, wl.for_ratio, 1.f / rsr_p,
@@ -355,13 +360,8 @@ UPBP_D float3 eval_bb1d(const QuerySeg& q, const StateWeights& cw, const Beam& l
     const float fpdf = (guided ? guide_pdf_at(q.o + q.d * tc, q.med, q.d, -lb.d, ph) : ph) * m.cont_prob;
     const float rpdf = ph * m.cont_prob;
     wc.d_shared *= tc * tc;
-    wc.d_shared /= rsf_c;
-    wc.d_bpt /= rsf_c;
-    wc.d_pde /= rsf_c;
-    wc.for_inv = 1.f / rsf_c;
-    wc.rev_inv = 1.f / rsr_c;
-    wc.for_ratio = ratio;
-    wc.rev_ratio = ratio;
+    wc.d_shared *= irf_c;
+    wc.d_pde *= irf_c;
     {
         // The reference multiplies by the squared distance from the beam's
         // origin, and not for first-segment beams of finite lights
@@ -372,25 +372,21 @@ UPBP_D float3 eval_bb1d(const QuerySeg& q, const StateWeights& cw, const Beam& l
         const float dl = tp + (p.mis_exact ? lb.origin_offset : 0.f);
         if (!skip) wl.d_shared *= dl * dl;
     }
-    wl.d_shared /= rsf_p;
-    wl.d_bpt /= rsf_p;
-    wl.d_pde /= rsf_p;
-    wl.for_inv = 1.f / rsf_p;
-    wl.rev_inv = 1.f / rsr_p;
-    wl.for_ratio = ratio;
-    wl.rev_ratio = ratio;
-    const float kernel = (1.f - bb_dist * bb_dist / p.radius_bb1d_2) * 3.f / (4.f * p.radius_bb1d * sin_theta);
+    wl.d_shared *= irf_p;
+    wl.d_pde *= irf_p;
+    const float inv_sin = 1.f / sin_theta;
+    const float kernel = (1.f - bb_dist * bb_dist * p.inv_radius_bb1d_2) * p.kernel_bb1d * inv_sin;
     if (!is_positive(kernel)) return v3(0.f);
     const float3 unweighted = lb.thr * m.scattering * att * f * kernel;
     if (is_black_or_negative(unweighted)) return v3(0.f);
-    const float ff = p.photon_beam_type == kLongBeam ? wl.for_inv : wl.for_ratio;
-    const float rf = p.camera_beam_type == kLongBeam ? wc.for_inv : wc.for_ratio;
-    const float val = 1.f / (p.mis_factor_bb1d * sin_theta * ff * rf);
+    const bool long_p = p.photon_beam_type == kLongBeam, long_c = p.camera_beam_type == kLongBeam;
+    const float ff = long_p ? irf_p : ratio, rf = long_c ? irf_c : ratio;
+    const float val = p.inv_mis_factor_bb1d * inv_sin * (long_p ? rsf_p : m.min_pos_att) * (long_c ? rsf_c : m.min_pos_att);
     const float bs = !wl.prev_specular;
-    const float w_light = val * (wl.d_shared * bs * p.subpath_count_bpt + fpdf * wl.d_pde / wl.rev_inv);
+    const float w_light = val * (wl.d_shared * bs * p.subpath_count_bpt + fpdf * wl.d_pde * rsr_p);
     const float w_local = 1.f + val * (p.mis_factor_bp2d * ff + p.mis_factor_pb2d * rf + p.mis_factor_pp3d);
     const float bt = !wc.prev_specular;
-    const float w_camera = val * (wc.d_shared * bt * p.subpath_count_bpt + rpdf * wc.d_pde / wc.rev_inv);
+    const float w_camera = val * (wc.d_shared * bt * p.subpath_count_bpt + rpdf * wc.d_pde * rsr_c);
     const float mis = 1.f / (w_light + w_local + w_camera);
     if (w_out) *w_out = mis;
     return mis * unweighted;

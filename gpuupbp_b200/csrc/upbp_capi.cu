@@ -1477,6 +1477,9 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             if (P.do_bb1d) P.rad_beam = std::max(P.rad_beam, r_bb1d);
             if (P.do_bp2d) P.rad_beam = std::max(P.rad_beam, r_bp2d);
             P.radius_bb1d_2 = r_bb1d * r_bb1d;
+            P.inv_radius_bb1d_2 = 1.f / P.radius_bb1d_2;
+            P.kernel_bb1d = 3.f / (4.f * r_bb1d);
+            P.inv_mis_factor_bb1d = 1.f / P.mis_factor_bb1d;
             P.radius_bp2d_2 = r_bp2d * r_bp2d;
             P.radius_pb2d_2 = r_pb2d * r_pb2d;
             P.radius_pp3d_2 = r_pp3d * r_pp3d;

@@ -354,6 +354,7 @@ struct DeviceParams {
     float radius_bb1d, radius_bp2d, radius_pb2d, radius_pp3d, radius_surf;
     float radius_bb1d_2, radius_bp2d_2, radius_pb2d_2, radius_pp3d_2, radius_surf_2;
     float rad_point_med, rad_beam;
+    float inv_radius_bb1d_2, kernel_bb1d, inv_mis_factor_bb1d;  // BB1D: 1 / r^2, 3 / (4 r), 1 / MIS factor
 
     // light-pass records
     LightVertexRec* vertices;
