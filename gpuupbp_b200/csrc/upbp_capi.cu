@@ -906,15 +906,19 @@ int sort_queries(upbp_ctx* c, int q, unsigned n, const unsigned** order)
     unsigned** b = c->d_sort[q];
     cub::DoubleBuffer<unsigned> kb(b[0], b[1]), vb(b[2], b[3]);
     size_t tb = c->sort_temp_bytes;
+    // Few queries: the upper bits alone, a pass of about 9 us for every 8
+    // (preview 64x64: 7 instead of 12 passes); their cells already hold less
+    // than one query on average, so the finer bits order next to nothing.
+    const int drop = n <= 16384u ? (q == 0 ? 36 : 6) : n <= 131072u ? (q == 0 ? 28 : 6) : 0;
     if (q == 0) {
         cub::DoubleBuffer<unsigned long long> kb64((unsigned long long*)b[0], (unsigned long long*)b[1]);
         PK(c).query_keys[1]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, kb64.Current(), nullptr, b[2]);
         UPBP_CK(cudaGetLastError());
-        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb64, vb, (int)n, 0, 60, c->st));
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb64, vb, (int)n, drop, 60, c->st));
     } else {
         PK(c).query_keys[0]<<<(n + 255) / 256, 256, 0, c->st>>>(c->slot, n, nullptr, b[0], b[2]);
         UPBP_CK(cudaGetLastError());
-        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb, vb, (int)n, 0, 30, c->st));
+        UPBP_CK(cub::DeviceRadixSort::SortPairs(c->d_sort_temp, tb, kb, vb, (int)n, drop, 30, c->st));
     }
     *order = vb.Current();
     return UPBP_OK;
