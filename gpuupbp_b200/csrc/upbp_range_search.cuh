@@ -115,13 +115,15 @@ struct PacketState {
     unsigned visits;            // of the warp
     unsigned cand, hits;        // of the lane
     bool overflow;
+    bool exact;                 // the round has one query
 };
 
 // Reserves the warp's next part of the hit list.  One atomic on the list's
 // total per 32 hits held the whole search to about two nanoseconds for each
 // (they all meet at one address): a warp that finds many pairs reserves ever
 // larger parts, up to 512 slots or a 2048th of the list, and marks at the end
-// what it did not use (a part is never larger than what it wrote before).
+// what it did not use.  A round of one query (`exact`) reserves by 32 only, so
+// that a list its pairs just fit is enough, as it was.
 UPBP_D void packet_reserve(PacketState& s, unsigned lane)
 {
     const DeviceParams& p = c_params;
@@ -130,7 +132,7 @@ UPBP_D void packet_reserve(PacketState& s, unsigned lane)
     s.at = __shfl_sync(~0u, base, 0);
     s.room = s.grab;
     s.seen = s.at + s.grab;
-    s.grab = min(2u * s.grab, max(32u, min(512u, p.hit_capacity >> 11 & ~31u)));
+    s.grab = s.exact ? 32u : min(2u * s.grab, max(32u, min(512u, p.hit_capacity >> 11 & ~31u)));
 }
 
 // Accepted pairs of up to 32 lanes, gathered by 32 for the hit list.
@@ -404,6 +406,7 @@ __global__ void __launch_bounds__(128, 7) range_search_kernel(int slot)
     s.grab = 32;
     s.visits = s.cand = s.hits = 0;
     s.overflow = false;
+    s.exact = n <= 1u;
     for (;;) {
         // no new queries once the hit list is 3/4 full, as far as this warp
         // saw at its last flush of hits
