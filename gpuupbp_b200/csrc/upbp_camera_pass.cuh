@@ -777,37 +777,61 @@ __global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
     }
 }
 
-// SURF and PP3D for one point-query record per thread, evaluated inline:
-// their walks are short and their hits few, so the search / evaluation split
-// (kept for PB2D, BB1D and BP2D) costs more than it saves here.
+// SURF and PP3D for one point-query record per thread: their walks are short
+// and their hits few, so the search / evaluation split (kept for PB2D, BB1D
+// and BP2D) costs more than it saves here.  A lane keeps the photons it finds
+// in shared memory, up to kPendingMerges, and the warp evaluates them together
+// (each lane its own, in the order found) when a lane's are full and at the
+// end: evaluated where they are found, about 60 merges of a warp at almost as
+// many different steps each ran on one or two lanes.
+constexpr unsigned kPendingMerges = 8;
+
 template <bool medium, bool kGuided>
-__global__ void __launch_bounds__(128) point_merge_kernel(int slot)
+__global__ void __launch_bounds__(128, 5) point_merge_kernel(int slot)
 {
     begin_kernel(medium ? kKernPp3d : kKernSurf, slot);
     const DeviceParams& p = c_params;
+    __shared__ unsigned s_found[kPendingMerges][128];
     const PointMap& map = medium ? p.med_map : p.surf_map;
     const float r2 = medium ? p.radius_pp3d_2 : p.radius_surf_2;
     const unsigned n = min(p.queue_count[1], p.pt_capacity);
-    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const unsigned k = p.pt_order ? __ldg(&p.pt_order[j]) : j;
-        const float4 q8 = __ldg(&p.pt_queue[k].q8);
-        if (!(fbits(q8.y) & (medium ? kQueryPp3d : kQuerySurf)) || !event_kept(fbits(q8.z), fbits(q8.w))) continue;
+    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; __any_sync(~0u, j < n); j += gridDim.x * blockDim.x) {
+        bool on = j < n;
+        unsigned k = 0;
+        float4 q8 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on) {
+            k = p.pt_order ? __ldg(&p.pt_order[j]) : j;
+            q8 = __ldg(&p.pt_queue[k].q8);
+            on = (fbits(q8.y) & (medium ? kQueryPp3d : kQuerySurf)) && event_kept(fbits(q8.z), fbits(q8.w));
+        }
+        if (!__any_sync(~0u, on)) continue;
         LightVertex cv;
-        load_vertex(&p.pt_queue[k].v, cv);
+        if (on) load_vertex(&p.pt_queue[k].v, cv);
         if (!kGuided) cv.bsdf.gcell = -1;  // the unguided instantiation has no proposal code
         float3 acc = v3(0.f);
-        points_in_radius(map, cv.hit, r2, [&](unsigned slot) {
-            LightVertex lv;
-            load_vertex(p.vertices + slot, lv);
-            float w = -1.f;
-            acc += eval_point_merge(lv, cv.path_length, cv.w, cv.bsdf, medium, &w);
-            UPBP_MISDBG(if (w >= 0.f) {
-                MisEvent e{medium ? kMisPp3d : kMisSurf, fbits(q8.z), cv.path_length, slot / p.slots_per_path,
-                           lv.path_length, 0u, w, lv.hit, cv.hit, 0.f, 0.f};
-                mis_event(e, nullptr, 0);
+        unsigned found = 0;
+        auto merge = [&]() {
+            for (unsigned i = 0; i < found; i++) {
+                const unsigned slot = s_found[i][threadIdx.x];
+                LightVertex lv;
+                load_vertex(p.vertices + slot, lv);
+                float w = -1.f;
+                acc += eval_point_merge(lv, cv.path_length, cv.w, cv.bsdf, medium, &w);
+                UPBP_MISDBG(if (w >= 0.f) {
+                    MisEvent e{medium ? kMisPp3d : kMisSurf, fbits(q8.z), cv.path_length, slot / p.slots_per_path,
+                               lv.path_length, 0u, w, lv.hit, cv.hit, 0.f, 0.f};
+                    mis_event(e, nullptr, 0);
+                });
+            }
+            found = 0;
+        };
+        points_in_radius_warp(
+            on, map, cv.hit, r2, [&](unsigned slot) { s_found[found++][threadIdx.x] = slot; },
+            [&]() {
+                if (__any_sync(~0u, found == kPendingMerges)) merge();
             });
-        });
-        splat_camera(fbits(q8.x), cv.thr * (medium ? p.pp3d_normalization : p.surf_normalization) * acc);
+        merge();
+        if (on) splat_camera(fbits(q8.x), cv.thr * (medium ? p.pp3d_normalization : p.surf_normalization) * acc);
     }
 }
 

@@ -33,6 +33,57 @@ UPBP_D void points_in_radius(const PointMap& map, float3 x, float r2, F&& f)
     if (!ok) flag_status(kErrTraversalStack);
 }
 
+// The same by a whole warp, one query per lane (`on` tells which lanes have
+// one): f as above, at most once a step, and step() by every lane after each
+// step of the walks.
+template <class F, class S>
+UPBP_D void points_in_radius_warp(bool on, const PointMap& map, float3 x, float r2, F&& f, S&& step)
+{
+    unsigned visits = 0, cand = 0, hits = 0;
+    bool ok = true;
+    int stack[kStackDepth];
+    int sp = 0;
+    int node = on && map.bvh.count > 0 ? (map.bvh.count > 1 ? 0 : ~0) : kWalkDone;
+    while (__any_sync(~0u, node != kWalkDone)) {
+        bool pop = false;
+        if (node >= 0) {
+            visits++;
+            const NodeBoxes nb = load_node(map.bvh.nodes, node);
+            const bool hl = inside(nb.llo, nb.lhi, x), hr = inside(nb.rlo, nb.rhi, x);
+            if (hl && hr) {
+                if (sp < kStackDepth)
+                    stack[sp++] = nb.r;
+                else
+                    ok = false;
+            }
+            if (hl || hr)
+                node = hl ? nb.l : nb.r;
+            else
+                pop = true;
+        }
+        if (!pop && node < 0 && node != kWalkDone) {
+            const int first = leaf_first(node), cnt = leaf_count(node);
+            const float4 pp = __ldg(&map.pos[first]);
+            cand++;
+            if (pred_point_point(x, xyz(pp), r2)) {
+                hits++;
+                f(fbits(pp.w));
+            }
+            if (cnt > 1)
+                node = leaf_link(first + 1, cnt - 1);
+            else
+                pop = true;
+        }
+        if (pop) node = sp > 0 ? stack[--sp] : kWalkDone;
+        step();
+    }
+    if (!on) return;
+    count_work(kCtrNodes, visits);
+    count_work(kCtrPointCand, cand);
+    count_work(kCtrPointHit, hits);
+    if (!ok) flag_status(kErrTraversalStack);
+}
+
 // Photons whose disc of radius r the query segment (o, d, (tmin, tmax))
 // crosses (PB2D): f(vertex slot, distance along the query, squared radius).
 template <class F>
