@@ -965,6 +965,19 @@ void range_search_split(DeviceParams& P, int mode)
     P.group_spread = mode == kModeBb1d ? 4.f * P.rad_beam : 6.f * (mode == kModePb2d ? P.rad_point_med : P.rad_beam);
 }
 
+// Most slots of a hit list of `capacity` entries that a warp of a search of
+// `blocks` blocks reserves at once: up to 512, and so few that all warps hold at
+// most an eighth of the list in reserve, which fits, with the pairs of the
+// queries in flight, the quarter a round keeps free.  (A 2048th of the list for
+// each of 4144 warps overflowed lists of up to 8.5M entries that could not grow
+// on empty slots alone: 9.6M pairs in a list of 4.2M took 12 searches and
+// evaluations beyond the first two, now 4.)  At 32 a part is reserved when 32
+// hits wait for it, and used whole.
+unsigned hit_reserve_limit(unsigned capacity, unsigned blocks)
+{
+    return std::max(32u, std::min(512u, capacity / (8u * kSearchWarps * blocks) & ~31u));
+}
+
 // Largest range-query hit list (8 bytes per entry, 34 GB, allocated only
 // when an iteration finds that many pairs); an iteration with more hits runs
 // its searches in rounds, each ending with a drain of the longest queries
@@ -1761,9 +1774,10 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 P.query_begin = begin;
                 P.query_end = end;
                 range_search_split(P, mode);
+                const unsigned g = cap_grid(c, (unsigned)c->search_grid[mode]);
+                P.hit_reserve = hit_reserve_limit(P.hit_capacity, g);
                 h2d += sizeof(P);
                 UPBP_CK(upload_params(c));
-                const int g = (int)cap_grid(c, (unsigned)c->search_grid[mode]);
                 switch (mode) {
                 case kModePb2d: PK(c).range_search[kModePb2d]<<<g, 128, 0, c->st>>>(c->slot); break;
                 case kModeBb1d: PK(c).range_search[kModeBb1d]<<<g, 128, 0, c->st>>>(c->slot); break;

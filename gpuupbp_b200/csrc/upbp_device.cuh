@@ -397,6 +397,7 @@ struct DeviceParams {
     unsigned query_begin, query_end;
     unsigned unit_max, units_per_warp;  // queries a warp takes at once (range_search_split)
     float group_spread;               // largest box of a group's start or end points
+    unsigned hit_reserve;             // most slots of the hit list a warp reserves at once (hit_reserve_limit)
     unsigned long long hit_soft_limit;
     HitState* hit_state;
 

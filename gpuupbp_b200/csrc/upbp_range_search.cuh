@@ -121,9 +121,9 @@ struct PacketState {
 // Reserves the warp's next part of the hit list.  One atomic on the list's
 // total per 32 hits held the whole search to about two nanoseconds for each
 // (they all meet at one address): a warp that finds many pairs reserves ever
-// larger parts, up to 512 slots or a 2048th of the list, and marks at the end
-// what it did not use.  A round of one query (`exact`) reserves by 32 only, so
-// that a list its pairs just fit is enough, as it was.
+// larger parts, up to hit_reserve slots, and marks at the end what it did not
+// use.  A round of one query (`exact`) reserves by 32 only, whatever the list,
+// so that a list its pairs just fit is enough.
 UPBP_D void packet_reserve(PacketState& s, unsigned lane)
 {
     const DeviceParams& p = c_params;
@@ -132,7 +132,7 @@ UPBP_D void packet_reserve(PacketState& s, unsigned lane)
     s.at = __shfl_sync(~0u, base, 0);
     s.room = s.grab;
     s.seen = s.at + s.grab;
-    s.grab = s.exact ? 32u : min(2u * s.grab, max(32u, min(512u, p.hit_capacity >> 11 & ~31u)));
+    s.grab = s.exact ? 32u : min(2u * s.grab, p.hit_reserve);
 }
 
 // Accepted pairs of up to 32 lanes, gathered by 32 for the hit list.
