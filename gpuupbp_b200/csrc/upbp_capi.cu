@@ -1605,8 +1605,10 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 alloc_ploc(c->ploc, nchunks + nchunks / 4);
             }
             if (!c->ploc_off && nchunks >= 2 && nchunks <= c->ploc.capacity) {
+                // as one cooperative launch it waits until all its blocks fit beside
+                // other jobs' kernels: the grid limit caps it too
                 UPBP_CK(build_ploc(src, nchunks, c->d_beam_nodes, c->sc, c->ploc, c->st, &order, &launches,
-                                   c->h_ploc, c->ploc_cap));
+                                   c->h_ploc, c->ploc_cap, c->grid_limit));
                 clustered = true;
                 c->ploc_pending = true;  // checked after the camera pass's synchronisation
                 c->ploc_src = src;
@@ -2054,6 +2056,20 @@ extern "C" int upbp_debug_scene_bvh(upbp_ctx* c, int real, float* nodes, uint64_
                                             cudaMemcpyDeviceToHost));
         if (tris && nt) UPBP_CK(cudaMemcpy(tris, g.tri, std::min(nt, tri_capacity) * sizeof(float),
                                            cudaMemcpyDeviceToHost));
+        return UPBP_OK;
+    });
+}
+
+// How the last iteration's beam map was built.
+extern "C" int upbp_debug_beam_map(upbp_ctx* c, uint32_t info[4])
+{
+    return upbp_host::abi_guard([&]() -> int {
+        if (!c || !info) return UPBP_ERR_ARGS;
+        const bool clustered = c->P.beam_map.bvh.count > 0 && c->beam_map_passes > 0;
+        info[0] = c->P.beam_map.bvh.count;
+        info[1] = clustered ? c->h_ploc[kPcPasses] : 0u;
+        info[2] = clustered ? c->h_ploc[kPcTailIters] : 0u;
+        info[3] = clustered ? c->ploc.blocks : 0u;
         return UPBP_OK;
     });
 }

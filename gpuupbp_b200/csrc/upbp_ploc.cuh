@@ -62,7 +62,8 @@ struct PlocScratch {
     unsigned* written = nullptr;   // writes per laid-out node index (the check)
     unsigned* order = nullptr;     // laid-out leaf order: chunk per leaf position
     unsigned* count = nullptr;     // kPcWords words
-    int grid = 0;                  // blocks of the clustering that are resident at once
+    int grid = 0;                  // blocks of the clustering's launch: what the device holds at once
+    unsigned blocks = 0;           // of the last build's launch
 };
 
 UPBP_D float ploc_area(float3 lo, float3 hi)
@@ -450,10 +451,11 @@ __global__ void k_ploc_check(unsigned n, const unsigned* written, unsigned* coun
 // ploc_complete after its next synchronisation with the stream, and until
 // then uses the tree for nothing; a tree that is not complete (the passes ran
 // out -- boxes so alike that few merge per pass -- or the layout check
-// failed) is replaced.
+// failed) is replaced.  The clustering takes at most max_blocks blocks (0: no
+// limit).
 inline cudaError_t build_ploc(const BoxSource& src, unsigned n, BvhNode* nodes, BuildScratch& sc, PlocScratch& ps,
                               cudaStream_t st, const unsigned** sorted_vals, unsigned* launches, unsigned* outcome,
-                              int passes)
+                              int passes, unsigned max_blocks)
 {
     passes = std::max(1, std::min(passes, kPlocPasses));
     if (n < 2 || n > ps.capacity || ps.grid < 1) return cudaErrorInvalidValue;
@@ -476,7 +478,9 @@ inline cudaError_t build_ploc(const BoxSource& src, unsigned n, BvhNode* nodes, 
     if (e != cudaSuccess) return e;
     k_ploc_init<<<grid, bs, 0, st>>>(src, vals, n, ps.cl[0], ps.leaf, ps.order);
     // one block per tile, no more than are resident at once (the grid barriers)
-    const unsigned blocks = std::min<unsigned>((unsigned)ps.grid, (n + kPlocBlock - 1) / kPlocBlock);
+    unsigned blocks = std::min<unsigned>((unsigned)ps.grid, (n + kPlocBlock - 1) / kPlocBlock);
+    if (max_blocks) blocks = std::min(blocks, max_blocks);
+    ps.blocks = blocks;
     void* args[] = {&n, &passes, &ps.cl[0], &ps.cl[1], &ps.act, &ps.block_sum, &ps.node_box, &ps.node_child,
                     &ps.node_up, &ps.count};
     e = cudaLaunchCooperativeKernel((const void*)k_ploc_cluster, dim3(blocks), dim3(kPlocBlock), args, 0, st);

@@ -122,7 +122,7 @@ EXPORTS = ["upbp_parse_command_line", "upbp_scene_load_obj", "upbp_scene_load_pr
            "upbp_write_image", "upbp_get_stream", "upbp_last_error",
            "upbp_debug_photons", "upbp_debug_query", "upbp_debug_query_static", "upbp_get_device",
            "upbp_debug_mis_records", "upbp_guide_info", "upbp_guide_gradients", "upbp_run_batch",
-           "upbp_set_grid_limit", "upbp_debug_scene_bvh", "upbp_save_checkpoint", "upbp_load_checkpoint"]
+           "upbp_set_grid_limit", "upbp_debug_scene_bvh", "upbp_debug_beam_map", "upbp_save_checkpoint", "upbp_load_checkpoint"]
 
 _libs = {}
 
@@ -166,6 +166,7 @@ def load_library(path: str = LIB_PATH):
     L.upbp_debug_query_static.argtypes = [VP, ctypes.c_int, VP, ctypes.c_uint32, VP, VP, ctypes.c_uint32]
     L.upbp_debug_scene_bvh.argtypes = [VP, ctypes.c_int, VP, ctypes.c_uint64, VP, ctypes.c_uint64,
                                        P(ctypes.c_uint32)]
+    L.upbp_debug_beam_map.argtypes = [VP, VP]
     L.upbp_save_checkpoint.argtypes = [VP, ctypes.c_char_p]
     L.upbp_load_checkpoint.argtypes = [VP, ctypes.c_char_p]
     _libs[path] = L
@@ -337,6 +338,12 @@ class Renderer:
         _check(self._L.upbp_debug_query(self._ctx, kind, q.ctypes.data, len(q), counts.ctypes.data,
                                                ids.ctypes.data, cap), "query")
         return [ids[i, :min(int(c), cap)].copy() for i, c in enumerate(counts)], counts
+
+    def beam_map(self) -> dict:
+        """How the last iteration's beam map was built (upbp_debug_beam_map)."""
+        info = np.zeros(4, np.uint32)
+        _check(self._L.upbp_debug_beam_map(self._ctx, info.ctypes.data), "beam map")
+        return dict(zip(("chunks", "passes", "tail_iterations", "blocks"), info.tolist()))
 
     def mis_records(self) -> dict:
         """MIS records of the last iteration (recording build only):

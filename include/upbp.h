@@ -335,6 +335,10 @@ int upbp_debug_scene_bvh(upbp_ctx* ctx, int real, float* nodes, uint64_t node_ca
                          uint64_t tri_capacity, uint32_t* count);
 int upbp_debug_query(upbp_ctx* ctx, int kind, const float* queries, uint32_t n, uint32_t* counts, uint32_t* ids,
                      uint32_t ids_per_query);
+/* upbp_debug_beam_map: the last iteration's beam map: its chunks (leaves),
+ * and of its clustering the many-cluster passes, the final block's
+ * iterations and the blocks of its launch (0 for the Morton-split LBVH). */
+int upbp_debug_beam_map(upbp_ctx* ctx, uint32_t info[4]);
 
 /* Same neighbour-set query as upbp_debug_query, for callers that cannot
  * allocate device memory per call (a fixed device-memory budget, or other
@@ -402,9 +406,10 @@ int upbp_guide_gradients(const float* params, uint32_t n_params, const float* x,
  * counter and drive each on the job's own stream and launch-parameter slot,
  * so one job's kernels and host synchronisations overlap the others' -- and
  * returns once every job's iteration is done: the OR of their status bits,
- * or the first job's error.  upbp_set_grid_limit caps the blocks of any of a
- * context's launches (0: no cap; the persistent kernels otherwise fill the
- * GPU), so that kernels of concurrent jobs share the SMs; the batch
+ * or the first job's error.  upbp_set_grid_limit caps the blocks of a
+ * context's passes, connections, range queries and beam-map clustering (0: no
+ * cap; these otherwise fill the GPU; the short sorts and copies around them
+ * are not capped), so that kernels of concurrent jobs share the SMs; the batch
  * autotuner in gpuupbp_b200/batch.py picks workers and the cap by timing. */
 int upbp_run_batch(upbp_ctx* const* ctxs, uint32_t n, int iteration, int workers);
 int upbp_set_grid_limit(upbp_ctx* ctx, uint32_t max_blocks);

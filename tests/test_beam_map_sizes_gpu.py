@@ -53,3 +53,31 @@ def test_sizes_span_the_tiles(scene_dir):
                             "-r_initial", "-0.02"], False)
         got.append(st["beam_chunks"])
     assert 0 < got[0] < 512 and 512 < got[1] < 2048 and got[2] > 4096
+
+
+def _blocks(scene_dir, env, limit):
+    from gpuupbp_b200 import upbp
+    path = scenes.write_workload("box_medium", scene_dir, tiny=True)
+    os.environ.update(env)  # read when the renderer is created
+    try:
+        r = upbp.Renderer(["-s", "-1", path, "-a", "upbp_bb1d+bp2d", "-l", "8", "-r", "33x29", "-pcpi", "4000",
+                           "-r_initial", "-0.02"])
+    finally:
+        for k in env:
+            os.environ.pop(k, None)
+    assert r._L.upbp_set_grid_limit(r._ctx, limit) == 0
+    status = r.run_iteration(1)
+    st, img, info = r.stats(), r.iteration_image().copy(), r.beam_map()
+    r.close()
+    return status, {k: st["work"][k]["beam_hit"] for k in ("bb1d_query", "bp2d_query")}, img, info
+
+
+@pytest.mark.parametrize("limit", [1, 3])
+def test_clustering_keeps_to_the_grid_limit(scene_dir, limit):
+    """The clustering's blocks, which have to be on the device all at once, are
+    capped like the other launches, and the map finds the same pairs."""
+    s0, hits0, img0, a = _blocks(scene_dir, {}, 0)
+    s1, hits1, img1, b = _blocks(scene_dir, {}, limit)
+    assert a["chunks"] == b["chunks"] > 4096 and a["blocks"] == -(-a["chunks"] // 512)  # one block a tile
+    assert b["blocks"] == limit and b["passes"] == a["passes"] > 0
+    assert s0 == s1 and hits0 == hits1 and np.allclose(img0, img1, rtol=1e-4, atol=1e-7)
