@@ -268,7 +268,8 @@ struct upbp_ctx {
     BoxSource ploc_src{};          // the build's source and size, to replace the tree
     unsigned ploc_n = 0;
     int ploc_cap = kPlocPasses;     // UPBP_PLOC_PASSES: at most this many
-    int ploc_failures = 0;          // builds that ran out of passes
+    unsigned ploc_blocks = 0;       // UPBP_PLOC_BLOCKS: blocks of the clustering's launch (0: as many as fit)
+    int ploc_failures = 0;          // builds that ran out of passes, or whose launch was refused
     bool ploc_off = false;  // UPBP_BEAM_MAP=lbvh: the beam map as a Morton-split LBVH
     void* d_scan_temp = nullptr;
     size_t scan_temp_bytes = 0;
@@ -832,17 +833,18 @@ void free_ploc(PlocScratch& ps)
 
 // Clustering scratch for cap leaves; on failure none (the beam map is then
 // built as an LBVH).
-void alloc_ploc(PlocScratch& ps, unsigned cap)
+void alloc_ploc(PlocScratch& ps, unsigned cap, unsigned blocks)
 {
     free_ploc(ps);
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0, per_sm = 0, cooperative = 0;
     const bool ok =
         cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && cooperative &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ploc_cluster, kPlocBlock, 0) == cudaSuccess &&
         sms * per_sm > 0 && dalloc(&ps.cl[0], 2 * (size_t)cap) == cudaSuccess &&
         dalloc(&ps.cl[1], 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.leaf, 2 * (size_t)cap) == cudaSuccess &&
-        dalloc(&ps.act, cap) == cudaSuccess && dalloc(&ps.block_sum, (size_t)sms * per_sm) == cudaSuccess &&
+        dalloc(&ps.act, cap) == cudaSuccess && dalloc(&ps.block_sum, std::max((size_t)sms * per_sm, (size_t)blocks)) == cudaSuccess &&
         dalloc(&ps.node_box, 2 * (size_t)cap) == cudaSuccess && dalloc(&ps.node_child, cap) == cudaSuccess &&
         dalloc(&ps.node_up, cap) == cudaSuccess && dalloc(&ps.written, cap) == cudaSuccess &&
         dalloc(&ps.order, cap) == cudaSuccess && dalloc(&ps.count, kPcWords) == cudaSuccess;
@@ -852,6 +854,7 @@ void alloc_ploc(PlocScratch& ps, unsigned cap)
         return;
     }
     ps.grid = sms * per_sm;
+    ps.forced = blocks;
     ps.capacity = cap;
 }
 
@@ -1264,6 +1267,7 @@ extern "C" int upbp_create(const upbp_scene_desc* s, const upbp_config* cfg, upb
             const int v = std::atoi(e);
             if (v > 0) c->ploc_cap = std::min(v, kPlocPasses);
         }
+        if (const char* e = std::getenv("UPBP_PLOC_BLOCKS")) c->ploc_blocks = (unsigned)std::max(0, std::atoi(e));
         if (const char* e = std::getenv("UPBP_MAX_HITS")) {
             const long long v = std::atoll(e);
             if (v > 0) c->max_hits = std::min<size_t>((size_t)v, kMaxHits);
@@ -1602,17 +1606,22 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             bool clustered = false;
             if (!c->ploc_off && nchunks > c->ploc.capacity) {
                 UPBP_CK(cudaStreamSynchronize(c->st));
-                alloc_ploc(c->ploc, nchunks + nchunks / 4);
+                alloc_ploc(c->ploc, nchunks + nchunks / 4, c->ploc_blocks);
             }
             if (!c->ploc_off && nchunks >= 2 && nchunks <= c->ploc.capacity) {
                 // as one cooperative launch it waits until all its blocks fit beside
                 // other jobs' kernels: the grid limit caps it too
-                UPBP_CK(build_ploc(src, nchunks, c->d_beam_nodes, c->sc, c->ploc, c->st, &order, &launches,
-                                   c->h_ploc, c->ploc_cap, c->grid_limit));
-                clustered = true;
-                c->ploc_pending = true;  // checked after the camera pass's synchronisation
-                c->ploc_src = src;
-                c->ploc_n = nchunks;
+                const cudaError_t pe = build_ploc(src, nchunks, c->d_beam_nodes, c->sc, c->ploc, c->st, &order,
+                                                  &launches, c->h_ploc, c->ploc_cap, c->grid_limit);
+                if (ploc_refused(pe)) {
+                    if (++c->ploc_failures >= 2) c->ploc_off = true;
+                } else {
+                    UPBP_CK(pe);
+                    clustered = true;
+                    c->ploc_pending = true;  // checked after the camera pass's synchronisation
+                    c->ploc_src = src;
+                    c->ploc_n = nchunks;
+                }
             }
             if (!clustered) {
                 c->beam_map_passes = 0;

@@ -63,6 +63,7 @@ struct PlocScratch {
     unsigned* order = nullptr;     // laid-out leaf order: chunk per leaf position
     unsigned* count = nullptr;     // kPcWords words
     int grid = 0;                  // blocks of the clustering's launch: what the device holds at once
+    unsigned forced = 0;           // UPBP_PLOC_BLOCKS: this many instead (more than fit are refused)
     unsigned blocks = 0;           // of the last build's launch
 };
 
@@ -452,7 +453,14 @@ __global__ void k_ploc_check(unsigned n, const unsigned* written, unsigned* coun
 // then uses the tree for nothing; a tree that is not complete (the passes ran
 // out -- boxes so alike that few merge per pass -- or the layout check
 // failed) is replaced.  The clustering takes at most max_blocks blocks (0: no
-// limit).
+// limit).  When the device refuses its cooperative launch (ploc_refused: too
+// many blocks for what it holds at once, or no such launches) there is no tree,
+// and the caller builds the LBVH instead.
+inline bool ploc_refused(cudaError_t e)
+{
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorLaunchOutOfResources;
+}
+
 inline cudaError_t build_ploc(const BoxSource& src, unsigned n, BvhNode* nodes, BuildScratch& sc, PlocScratch& ps,
                               cudaStream_t st, const unsigned** sorted_vals, unsigned* launches, unsigned* outcome,
                               int passes, unsigned max_blocks)
@@ -479,12 +487,16 @@ inline cudaError_t build_ploc(const BoxSource& src, unsigned n, BvhNode* nodes, 
     k_ploc_init<<<grid, bs, 0, st>>>(src, vals, n, ps.cl[0], ps.leaf, ps.order);
     // one block per tile, no more than are resident at once (the grid barriers)
     unsigned blocks = std::min<unsigned>((unsigned)ps.grid, (n + kPlocBlock - 1) / kPlocBlock);
+    if (ps.forced) blocks = ps.forced;
     if (max_blocks) blocks = std::min(blocks, max_blocks);
     ps.blocks = blocks;
     void* args[] = {&n, &passes, &ps.cl[0], &ps.cl[1], &ps.act, &ps.block_sum, &ps.node_box, &ps.node_child,
                     &ps.node_up, &ps.count};
     e = cudaLaunchCooperativeKernel((const void*)k_ploc_cluster, dim3(blocks), dim3(kPlocBlock), args, 0, st);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // a refused launch is not sticky
+        return e;
+    }
     k_ploc_place<<<grid, bs, 0, st>>>(n, ps.leaf, vals, ps.node_box, ps.node_child, ps.node_up, ps.written, ps.order,
                                       nodes, ps.count);
     k_ploc_check<<<std::min(grid, 1184u), bs, 0, st>>>(n, ps.written, ps.count);

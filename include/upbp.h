@@ -249,8 +249,8 @@ typedef struct upbp_stats {
     /* Clustering passes (many-cluster passes and the final block's
      * iterations) that built the last iteration's beam map; 0: the
      * Morton-split LBVH (UPBP_BEAM_MAP=lbvh, or the clustering fell back:
-     * its passes ran out -- UPBP_PLOC_PASSES caps them -- or its layout
-     * check failed). */
+     * its passes ran out -- UPBP_PLOC_PASSES caps them --, its layout check
+     * failed, or the device refused its cooperative launch). */
     uint32_t beam_map_passes;
 } upbp_stats;
 

@@ -81,3 +81,12 @@ def test_clustering_keeps_to_the_grid_limit(scene_dir, limit):
     assert a["chunks"] == b["chunks"] > 4096 and a["blocks"] == -(-a["chunks"] // 512)  # one block a tile
     assert b["blocks"] == limit and b["passes"] == a["passes"] > 0
     assert s0 == s1 and hits0 == hits1 and np.allclose(img0, img1, rtol=1e-4, atol=1e-7)
+
+
+def test_refused_clustering_falls_back(scene_dir):
+    """More blocks than the device holds at once: the runtime refuses the
+    launch, and the iteration renders with the LBVH."""
+    s0, hits0, img0, a = _blocks(scene_dir, {}, 0)
+    s1, hits1, img1, b = _blocks(scene_dir, {"UPBP_PLOC_BLOCKS": "65536"}, 0)
+    assert a["blocks"] > 0 and b == {"chunks": a["chunks"], "passes": 0, "tail_iterations": 0, "blocks": 0}
+    assert s0 == s1 and hits0 == hits1 and np.allclose(img0, img1, rtol=1e-4, atol=1e-7)
