@@ -1584,8 +1584,10 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
         }
         if ((P.build_bb1d || P.build_bp2d) && nb > 0) {
             // split beams into chunks of about 6 beam radii, at most 64 per beam
+            // (fewer where their sum could wrap)
             const float chunk_len = 6.f * P.rad_beam;
-            k_chunk_counts<<<(nb + 255) / 256, 256, 0, c->st>>>(c->d_beams, nb, chunk_len, 64u, c->d_chunk_counts);
+            k_chunk_counts<<<(nb + 255) / 256, 256, 0, c->st>>>(c->d_beams, nb, chunk_len,
+                                                                std::min(64u, 0xffffffffu / nb), c->d_chunk_counts);
             size_t tb = c->scan_temp_bytes;
             UPBP_CK(cub::DeviceScan::ExclusiveSum(c->d_scan_temp, tb, c->d_chunk_counts, c->d_chunk_offsets, (int)nb, c->st));
             unsigned tail[2] = {0, 0};
@@ -1594,6 +1596,11 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             UPBP_CK(cudaMemcpyAsync(&tail[1], c->d_chunk_counts + nb - 1, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
             UPBP_CK(cudaStreamSynchronize(c->st));
             const unsigned nchunks = tail[0] + tail[1];
+            if (nchunks > kMaxBvhPrimitives) {
+                upbp_host::set_error("beam map of " + std::to_string(nchunks) + " chunks: at most " +
+                                     std::to_string(kMaxBvhPrimitives));
+                return UPBP_ERR_CUDA;
+            }
             if (ensure_chunks(c, nchunks) != UPBP_OK) return UPBP_ERR_CUDA;
             P.beam_map = BeamMap{BvhView{c->d_beam_nodes, 0, c->d_beam_qnodes}, c->d_beam_leaf, c->d_beams, beam_dilate};
             k_chunk_expand<<<(nb + 255) / 256, 256, 0, c->st>>>(c->d_chunk_counts, c->d_chunk_offsets, nb, c->d_chunks);

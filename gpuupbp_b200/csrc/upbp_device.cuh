@@ -121,6 +121,7 @@ struct __align__(16) QNode4 {
 // Link bits beside the index: which of its two children are leaves, or that
 // it is a single leaf.
 enum : unsigned { kQnodeLeaf0 = 1u << 28, kQnodeLeaf1 = 1u << 29, kQnodeSingle = 1u << 30 };
+static_assert(kMaxBvhPrimitives <= kQnodeLeaf0, "a link's index fits below its bits");
 
 // Step 2^(e - 127) of a biased exponent byte e in 1..254.
 UPBP_D float qnode_step(unsigned e) { return __uint_as_float(e << 23); }

@@ -466,7 +466,8 @@ inline cudaError_t build_ploc(const BoxSource& src, unsigned n, BvhNode* nodes, 
                               int passes, unsigned max_blocks)
 {
     passes = std::max(1, std::min(passes, kPlocPasses));
-    if (n < 2 || n > ps.capacity || ps.grid < 1) return cudaErrorInvalidValue;
+    // (leaf links hold kLeafShift bits, and so do the searches' entries)
+    if (n < 2 || n > kMaxBvhPrimitives || n > ps.capacity || ps.grid < 1) return cudaErrorInvalidValue;
     // Morton order of the centres
     const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     cudaError_t e = cudaMemcpyAsync(sc.ord6, init, sizeof(init), cudaMemcpyHostToDevice, st);
