@@ -154,10 +154,9 @@ UPBP_D bool bvh_walk(const BvhView& bvh, BoxTest&& test_box, Leaf&& leaf)
     }
 }
 
-// Resumable form of bvh_walk: walk_step() advances by exactly one internal
-// node or one leaf, so a warp can move all its lanes in lock step and give a
-// lane that finished its query a new one (the range-query search kernels).
-// Visits the same leaves in the same order as bvh_walk.
+// Resumable form of bvh_walk (beams_near_segment): walk_step() advances by
+// exactly one internal node or one leaf.  Visits the same leaves in the same
+// order as bvh_walk.
 constexpr int kWalkDone = INT_MIN;
 
 struct WalkState {

@@ -785,13 +785,33 @@ __global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
 // end: evaluated where they are found, about 60 merges of a warp at almost as
 // many different steps each ran on one or two lanes.
 constexpr unsigned kPendingMerges = 8;
+constexpr int kMergeThreads = 128;  // of the blocks that merge points
+
+// merge(slot), on the query's lane, for every photon within the radius of x.
+template <class F>
+UPBP_D void merge_points(bool on, const PointMap& map, float3 x, float r2, F&& merge)
+{
+    __shared__ unsigned s_found[kPendingMerges][kMergeThreads];
+    unsigned found = 0, merged = 0;
+    auto flush = [&]() {
+        for (unsigned i = 0; i < found; i++) merge(s_found[i][threadIdx.x]);
+        merged += found;
+        found = 0;
+    };
+    points_in_radius_warp(
+        on, map, x, r2, [&](unsigned slot) { s_found[found++][threadIdx.x] = slot; },
+        [&]() {
+            if (__any_sync(~0u, found == kPendingMerges)) flush();
+        });
+    flush();
+    if (on) count_work(kCtrPointHit, merged);
+}
 
 template <bool medium, bool kGuided>
-__global__ void __launch_bounds__(128, 5) point_merge_kernel(int slot)
+__global__ void __launch_bounds__(kMergeThreads, 5) point_merge_kernel(int slot)
 {
     begin_kernel(medium ? kKernPp3d : kKernSurf, slot);
     const DeviceParams& p = c_params;
-    __shared__ unsigned s_found[kPendingMerges][128];
     const PointMap& map = medium ? p.med_map : p.surf_map;
     const float r2 = medium ? p.radius_pp3d_2 : p.radius_surf_2;
     const unsigned n = min(p.queue_count[1], p.pt_capacity);
@@ -809,28 +829,17 @@ __global__ void __launch_bounds__(128, 5) point_merge_kernel(int slot)
         if (on) load_vertex(&p.pt_queue[k].v, cv);
         if (!kGuided) cv.bsdf.gcell = -1;  // the unguided instantiation has no proposal code
         float3 acc = v3(0.f);
-        unsigned found = 0;
-        auto merge = [&]() {
-            for (unsigned i = 0; i < found; i++) {
-                const unsigned slot = s_found[i][threadIdx.x];
-                LightVertex lv;
-                load_vertex(p.vertices + slot, lv);
-                float w = -1.f;
-                acc += eval_point_merge(lv, cv.path_length, cv.w, cv.bsdf, medium, &w);
-                UPBP_MISDBG(if (w >= 0.f) {
-                    MisEvent e{medium ? kMisPp3d : kMisSurf, fbits(q8.z), cv.path_length, slot / p.slots_per_path,
-                               lv.path_length, 0u, w, lv.hit, cv.hit, 0.f, 0.f};
-                    mis_event(e, nullptr, 0);
-                });
-            }
-            found = 0;
-        };
-        points_in_radius_warp(
-            on, map, cv.hit, r2, [&](unsigned slot) { s_found[found++][threadIdx.x] = slot; },
-            [&]() {
-                if (__any_sync(~0u, found == kPendingMerges)) merge();
+        merge_points(on, map, cv.hit, r2, [&](unsigned slot) {
+            LightVertex lv;
+            load_vertex(p.vertices + slot, lv);
+            float w = -1.f;
+            acc += eval_point_merge(lv, cv.path_length, cv.w, cv.bsdf, medium, &w);
+            UPBP_MISDBG(if (w >= 0.f) {
+                MisEvent e{medium ? kMisPp3d : kMisSurf, fbits(q8.z), cv.path_length, slot / p.slots_per_path,
+                           lv.path_length, 0u, w, lv.hit, cv.hit, 0.f, 0.f};
+                mis_event(e, nullptr, 0);
             });
-        merge();
+        });
         if (on) splat_camera(fbits(q8.x), cv.thr * (medium ? p.pp3d_normalization : p.surf_normalization) * acc);
     }
 }

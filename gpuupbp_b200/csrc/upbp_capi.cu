@@ -170,7 +170,8 @@ cudaError_t dupload(T** p, const T* h, size_t n, cudaStream_t st)
     return cudaMemcpyAsync(*p, h, n * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
-// Neighbour sets of n queries through the estimators' range-query walkers.
+// Neighbour sets of n queries by a walk per query through the uncompressed
+// nodes of the maps (upbp_queries.cuh), apart from the searches that render.
 // Query record: x y z dx dy dz tmin tmax (points use x y z only).
 __global__ void k_debug_query(int slot, int kind, const float* q, unsigned n, unsigned* counts, unsigned* ids,
                               unsigned cap)
@@ -206,6 +207,56 @@ __global__ void k_debug_query(int slot, int kind, const float* q, unsigned n, un
         break;
     }
     counts[i] = k;
+}
+
+// Query records of the renderer's own searches for n such queries: segment
+// records without a medium filter, point records of one path.
+__global__ void k_debug_records(const float* q, unsigned n, SegQueryRec* seg, PointQueryRec* pt)
+{
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float* r = q + 8 * (size_t)i;
+    if (seg) {
+        seg[i].q[0] = make_float4(r[0], r[1], r[2], r[6]);
+        seg[i].q[1] = make_float4(r[3], r[4], r[5], r[7]);
+        seg[i].q[2] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+    } else {
+        pt[i].v.q[0] = make_float4(r[0], r[1], r[2], 0.f);
+        pt[i].q8 = make_float4(0.f, __uint_as_float(kQueryBp2d), 0.f, 0.f);  // path 0, event key 0
+    }
+}
+
+// The pairs of a hit list as neighbour sets.
+__global__ void k_debug_collect(const uint2* hits, unsigned long long total, unsigned* counts, unsigned* ids,
+                                unsigned cap)
+{
+    for (unsigned long long j = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; j < total;
+         j += (unsigned long long)gridDim.x * blockDim.x) {
+        const uint2 h = hits[j];
+        if (h.x == kNoHit) continue;
+        const unsigned k = atomicAdd(&counts[h.x], 1u);
+        if (k < cap) ids[(size_t)h.x * cap + k] = h.y;
+    }
+}
+
+// Neighbour sets through the merging walk of SURF and PP3D.
+template <bool medium>
+__global__ void __launch_bounds__(kMergeThreads) k_debug_merge(int slot, const float* q, unsigned n, unsigned* counts,
+                                                               unsigned* ids, unsigned cap)
+{
+    begin_kernel(kKernDebug, slot);
+    const DeviceParams& p = c_params;
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = i < n;
+    if (!__any_sync(~0u, on)) return;
+    const float* r = q + 8 * (size_t)(on ? i : 0u);
+    unsigned k = 0;
+    merge_points(on, medium ? p.med_map : p.surf_map, make_float3(r[0], r[1], r[2]),
+                 medium ? p.radius_pp3d_2 : p.radius_surf_2, [&](unsigned id) {
+                     if (k < cap) ids[(size_t)i * cap + k] = id;
+                     k++;
+                 });
+    if (on) counts[i] = k;
 }
 
 }  // namespace
@@ -1019,6 +1070,76 @@ int ensure_hits(upbp_ctx* c, size_t n)
     return UPBP_OK;
 }
 
+// Searches the first nq queries of a range query's queue into the hit list,
+// in rounds over their order, and calls evaluate(total) -- launches on the
+// context's stream -- on the list of each round.  A round stops handing out
+// queries when the list is 3/4 full; if the queries in flight then overflow
+// it, the round is repeated (the search is a pure function of the queries and
+// the map) with a larger list or a shorter range.  `found` receives the slots
+// used.
+template <class Evaluate>
+int search_rounds(upbp_ctx* c, int mode, unsigned nq, unsigned& launches, size_t& h2d, size_t& d2h,
+                  unsigned long long& found, Evaluate&& evaluate)
+{
+    DeviceParams& P = c->P;
+    static constexpr int kKern[kRangeModes] = {kKernPb2d, kKernBb1d, kKernBp2d};
+    unsigned long long* work = P.work + (size_t)kKern[mode] * kCtrCount;
+    const size_t work_bytes = kCtrCount * sizeof(unsigned long long);
+    UPBP_CK(cudaMemsetAsync(work, 0, work_bytes, c->st));
+    unsigned begin = 0, span = nq;  // span: longest range of a round, halved after an overflow
+    int repeats = 0;
+    while (begin < nq) {
+        const unsigned end = begin + std::min(span, nq - begin);
+        UPBP_CK(cudaMemsetAsync(c->d_hit_state, 0, sizeof(HitState), c->st));
+        UPBP_CK(cudaMemcpyAsync(c->d_work_saved, work, work_bytes, cudaMemcpyDeviceToDevice, c->st));
+        P.hit_qb = c->d_hit_qb;
+        P.hit_capacity = c->hit_capacity;
+        P.hit_soft_limit = c->hit_capacity - c->hit_capacity / 4;
+        P.query_begin = begin;
+        P.query_end = end;
+        const unsigned g = cap_grid(c, (unsigned)c->search_grid[mode]);
+        P.hit_reserve = hit_reserve_limit(P.hit_capacity, g);
+        h2d += sizeof(P);
+        UPBP_CK(upload_params(c));
+        switch (mode) {
+        case kModePb2d: PK(c).range_search[kModePb2d]<<<g, 128, 0, c->st>>>(c->slot); break;
+        case kModeBb1d: PK(c).range_search[kModeBb1d]<<<g, 128, 0, c->st>>>(c->slot); break;
+        default: PK(c).range_search[kModeBp2d]<<<g, 128, 0, c->st>>>(c->slot); break;
+        }
+        launches++;
+        UPBP_CK(cudaGetLastError());
+        d2h += sizeof(HitState);
+        UPBP_CK(cudaMemcpyAsync(&c->h_hit_state, c->d_hit_state, sizeof(HitState), cudaMemcpyDeviceToHost, c->st));
+        UPBP_CK(cudaStreamSynchronize(c->st));
+        const unsigned long long total = c->h_hit_state.total;
+        const unsigned done = (unsigned)std::min<unsigned long long>(c->h_hit_state.fetched, end - begin);
+        if (total > c->hit_capacity || done == 0) {
+            if (++repeats > 64) {  // repeats of one round
+                upbp_host::set_error("range search made no progress");
+                return UPBP_ERR_CUDA;
+            }
+            UPBP_CK(cudaMemcpyAsync(work, c->d_work_saved, work_bytes, cudaMemcpyDeviceToDevice, c->st));
+            if (c->hit_capacity < c->max_hits) {
+                if (ensure_hits(c, (size_t)std::min<unsigned long long>(total, c->max_hits)) != UPBP_OK)
+                    return UPBP_ERR_CUDA;
+            } else {
+                span = std::max(1u, std::min(done, end - begin) / 2);
+            }
+            continue;
+        }
+        if (total > 0) {
+            evaluate(total);
+            launches++;
+            UPBP_CK(cudaGetLastError());
+        }
+        found += total;
+        begin += done;
+        repeats = 0;
+        span = span > nq / 2 ? nq : 2 * span;
+    }
+    return UPBP_OK;
+}
+
 }  // namespace
 
 // ---- neighbour-set query without device allocation --------------------
@@ -1767,93 +1888,39 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             UPBP_CK(upload_params(c));
         }
         // The estimators: search (query, neighbour) pairs into the hit list, then
-        // evaluate them, in rounds over the query order.  A round stops handing
-        // out queries when the list is 3/4 full; if the queries in flight then
-        // overflow it, the round is repeated (the search is a pure function of
-        // the queries and the map) with a larger list or a shorter range.  A list
-        // that needed more than one round is grown for the next estimator and
-        // iteration (up to max_hits).
+        // evaluate them, in rounds (search_rounds).  A list that needed more than
+        // one round is grown for the next estimator and iteration (up to
+        // max_hits).
         auto estimator = [&](int mode, unsigned nq) -> int {
-            static constexpr int kKern[kRangeModes] = {kKernPb2d, kKernBb1d, kKernBp2d};
-            unsigned long long* work = c->d_work + (size_t)kKern[mode] * kCtrCount;
-            const size_t work_bytes = kCtrCount * sizeof(unsigned long long);
             if (c->hit_capacity == 0 && ensure_hits(c, (size_t)std::max(nseg, npt) * 32) != UPBP_OK) return UPBP_ERR_CUDA;
-            UPBP_CK(cudaMemsetAsync(work, 0, work_bytes, c->st));
+            range_search_split(P, mode);
             unsigned long long found = 0;
-            unsigned begin = 0, span = nq;  // span: longest range of a round, halved after an overflow
-            int repeats = 0;
-            while (begin < nq) {
-                const unsigned end = begin + std::min(span, nq - begin);
-                UPBP_CK(cudaMemsetAsync(c->d_hit_state, 0, sizeof(HitState), c->st));
-                UPBP_CK(cudaMemcpyAsync(c->d_work_saved, work, work_bytes, cudaMemcpyDeviceToDevice, c->st));
-                P.hit_qb = c->d_hit_qb;
-                P.hit_capacity = c->hit_capacity;
-                P.hit_soft_limit = c->hit_capacity - c->hit_capacity / 4;
-                P.query_begin = begin;
-                P.query_end = end;
-                range_search_split(P, mode);
-                const unsigned g = cap_grid(c, (unsigned)c->search_grid[mode]);
-                P.hit_reserve = hit_reserve_limit(P.hit_capacity, g);
-                h2d += sizeof(P);
-                UPBP_CK(upload_params(c));
+            const int rc = search_rounds(c, mode, nq, launches, h2d, d2h, found, [&](unsigned long long total) {
+                // no more blocks than are resident: the blocks then sweep
+                // the list once, side by side, and the records of the
+                // pairs in flight (neighbours in the list share queries
+                // and nearby beams) stay in L2; with more blocks every
+                // wave of resident blocks swept the whole list and read
+                // the records again
+                const unsigned g2 = cap_grid(
+                    c, std::max(1u, std::min<unsigned>((unsigned)((total + 127) / 128), (unsigned)c->eval_grid[mode])));
+                const bool gd = P.guide.entries != nullptr;
                 switch (mode) {
-                case kModePb2d: PK(c).range_search[kModePb2d]<<<g, 128, 0, c->st>>>(c->slot); break;
-                case kModeBb1d: PK(c).range_search[kModeBb1d]<<<g, 128, 0, c->st>>>(c->slot); break;
-                default: PK(c).range_search[kModeBp2d]<<<g, 128, 0, c->st>>>(c->slot); break;
+                case kModePb2d:
+                    if (gd) PK(c).range_eval[kModePb2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModePb2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    break;
+                case kModeBb1d:
+                    if (gd) PK(c).range_eval[kModeBb1d][1]<<<g2, 128, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModeBb1d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    break;
+                default:
+                    if (gd) PK(c).range_eval[kModeBp2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModeBp2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    break;
                 }
-                launches++;
-                UPBP_CK(cudaGetLastError());
-                d2h += sizeof(HitState);
-                UPBP_CK(cudaMemcpyAsync(&c->h_hit_state, c->d_hit_state, sizeof(HitState), cudaMemcpyDeviceToHost, c->st));
-                UPBP_CK(cudaStreamSynchronize(c->st));
-                const unsigned long long total = c->h_hit_state.total;
-                const unsigned done = (unsigned)std::min<unsigned long long>(c->h_hit_state.fetched, end - begin);
-                if (total > c->hit_capacity || done == 0) {
-                    if (++repeats > 64) {  // repeats of one round
-                        upbp_host::set_error("range search made no progress");
-                        return UPBP_ERR_CUDA;
-                    }
-                    UPBP_CK(cudaMemcpyAsync(work, c->d_work_saved, work_bytes, cudaMemcpyDeviceToDevice, c->st));
-                    if (c->hit_capacity < c->max_hits) {
-                        if (ensure_hits(c, (size_t)std::min<unsigned long long>(total, c->max_hits)) != UPBP_OK)
-                            return UPBP_ERR_CUDA;
-                    } else {
-                        span = std::max(1u, std::min(done, end - begin) / 2);
-                    }
-                    continue;
-                }
-                if (total > 0) {
-                    // no more blocks than are resident: the blocks then sweep
-                    // the list once, side by side, and the records of the
-                    // pairs in flight (neighbours in the list share queries
-                    // and nearby beams) stay in L2; with more blocks every
-                    // wave of resident blocks swept the whole list and read
-                    // the records again
-                    const unsigned g2 = cap_grid(
-                        c, std::max(1u, std::min<unsigned>((unsigned)((total + 127) / 128), (unsigned)c->eval_grid[mode])));
-                    const bool gd = P.guide.entries != nullptr;
-                    switch (mode) {
-                    case kModePb2d:
-                        if (gd) PK(c).range_eval[kModePb2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                        else PK(c).range_eval[kModePb2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
-                        break;
-                    case kModeBb1d:
-                        if (gd) PK(c).range_eval[kModeBb1d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                        else PK(c).range_eval[kModeBb1d][0]<<<g2, 128, 0, c->st>>>(c->slot);
-                        break;
-                    default:
-                        if (gd) PK(c).range_eval[kModeBp2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                        else PK(c).range_eval[kModeBp2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
-                        break;
-                    }
-                    launches++;
-                    UPBP_CK(cudaGetLastError());
-                }
-                found += total;
-                begin += done;
-                repeats = 0;
-                span = span > nq / 2 ? nq : 2 * span;
-            }
+            });
+            if (rc != UPBP_OK) return rc;
             if (found > c->hit_capacity - c->hit_capacity / 4 &&
                 ensure_hits(c, (size_t)std::min<unsigned long long>(found + found / 8, c->max_hits)) != UPBP_OK)
                 return UPBP_ERR_CUDA;
@@ -1861,14 +1928,14 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
         };
         UPBP_CK(cudaEventRecord(ev[6], c->st));
         if (run_surf) {
-            if (P.guide.entries) PK(c).point_merge[0][1]<<<grid_for(npt), 128, 0, c->st>>>(c->slot);
-            else PK(c).point_merge[0][0]<<<grid_for(npt), 128, 0, c->st>>>(c->slot);
+            if (P.guide.entries) PK(c).point_merge[0][1]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
+            else PK(c).point_merge[0][0]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         UPBP_CK(cudaEventRecord(ev[7], c->st));
         if (run_pp3d) {
-            if (P.guide.entries) PK(c).point_merge[1][1]<<<grid_for(npt), 128, 0, c->st>>>(c->slot);
-            else PK(c).point_merge[1][0]<<<grid_for(npt), 128, 0, c->st>>>(c->slot);
+            if (P.guide.entries) PK(c).point_merge[1][1]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
+            else PK(c).point_merge[1][0]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         UPBP_CK(cudaEventRecord(ev[8], c->st));
@@ -2150,6 +2217,97 @@ extern "C" int upbp_debug_query_static(upbp_ctx* c, int kind, const float* queri
         UPBP_CK(cudaGetLastError());
         UPBP_CK(cudaMemcpyAsync(counts, dc, n * sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
         if (ids && id_bytes) UPBP_CK(cudaMemcpyAsync(ids, di, id_bytes, cudaMemcpyDeviceToHost, c->st));
+        UPBP_CK(cudaStreamSynchronize(c->st));
+        return UPBP_OK;
+    });
+}
+
+// Neighbour sets of n queries through the searches that render: the range
+// searches of PB2D, BB1D and BP2D with their rounds and hit list, the merging
+// walk of SURF and PP3D.
+extern "C" int upbp_debug_search(upbp_ctx* c, int kind, const float* queries, uint32_t n, uint32_t unit_max,
+                                 float group_spread, uint32_t* counts, uint32_t* ids, uint32_t ids_per_query)
+{
+    return upbp_host::abi_guard([&]() -> int {
+        if (!c || !queries || !counts || kind < 0 || kind > 4 || unit_max > 32 || (unit_max & (unit_max - 1)) ||
+            n >= kNoHit)
+            return UPBP_ERR_ARGS;
+        if (kind == 2 || kind == 3)
+            for (uint32_t i = 0; i < n; i++) {
+                const float* d = queries + 8 * (size_t)i + 3;
+                if (!(std::fabs(d[0] * d[0] + d[1] * d[1] + d[2] * d[2] - 1.f) < 1e-5f)) {
+                    upbp_host::set_error("upbp_debug_search: a direction is not of unit length");
+                    return UPBP_ERR_ARGS;
+                }
+            }
+        if (n == 0) return UPBP_OK;
+        DeviceGuard dg(c->dev);
+        UPBP_CK(dg.error());
+        // the call's buffers, and the context's parameters as they were
+        struct Call {
+            upbp_ctx* c;
+            const DeviceParams keep;
+            float* q = nullptr;
+            unsigned *counts = nullptr, *ids = nullptr, *words = nullptr;
+            SegQueryRec* seg = nullptr;
+            PointQueryRec* pt = nullptr;
+            unsigned long long* work = nullptr;
+            explicit Call(upbp_ctx* ctx) : c(ctx), keep(ctx->P) {}
+            ~Call()
+            {
+                cudaStreamSynchronize(c->st);
+                void* b[] = {q, counts, ids, words, seg, pt, work};
+                for (void* x : b) cudaFree(x);
+                c->P = keep;
+            }
+        } t(c);
+        const size_t id_bytes = (size_t)n * ids_per_query * sizeof(unsigned);
+        UPBP_CK(dalloc(&t.q, 8 * (size_t)n));
+        UPBP_CK(dalloc(&t.counts, n));
+        UPBP_CK(dalloc(&t.ids, (size_t)n * std::max(1u, ids_per_query)));
+        UPBP_CK(dalloc(&t.words, 3));
+        UPBP_CK(dalloc(&t.work, (size_t)kKernRows * kCtrCount));  // the iteration's own counters stay
+        UPBP_CK(cudaMemcpyAsync(t.q, queries, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->st));
+        UPBP_CK(cudaMemsetAsync(t.counts, 0, n * sizeof(unsigned), c->st));
+        UPBP_CK(cudaMemsetAsync(t.work, 0, (size_t)kKernRows * kCtrCount * sizeof(unsigned long long), c->st));
+        const unsigned words[3] = {n, n, 0xffffffffu};  // both queues' lengths; path 0: no failed step
+        UPBP_CK(cudaMemcpyAsync(t.words, words, sizeof(words), cudaMemcpyHostToDevice, c->st));
+        DeviceParams& P = c->P;
+        P.work = t.work;
+        SlotLease lease(c->dev, c->slot, c->st);
+        if (kind < 2) {
+            UPBP_CK(upload_params(c));
+            const unsigned g = (n + kMergeThreads - 1) / kMergeThreads;
+            if (kind == 0) k_debug_merge<false><<<g, kMergeThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
+            else k_debug_merge<true><<<g, kMergeThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
+            UPBP_CK(cudaGetLastError());
+        } else if ((kind == 2 ? P.med_map.bvh.count : P.beam_map.bvh.count) > 0) {
+            const int mode = kind == 2 ? kModePb2d : kind == 3 ? kModeBb1d : kModeBp2d;
+            if (kind == 4) UPBP_CK(dalloc(&t.pt, n));
+            else UPBP_CK(dalloc(&t.seg, n));
+            k_debug_records<<<(n + 127) / 128, 128, 0, c->st>>>(t.q, n, t.seg, t.pt);
+            UPBP_CK(cudaGetLastError());
+            P.seg_queue = t.seg;
+            P.pt_queue = t.pt;
+            P.seg_capacity = P.pt_capacity = n;
+            P.seg_order = P.pt_order = nullptr;
+            P.queue_count = t.words;
+            P.path_err = t.words + 2;
+            range_search_split(P, mode);
+            if (unit_max) P.unit_max = unit_max;
+            if (group_spread > 0.f) P.group_spread = group_spread;
+            HitLease hits(c);
+            if (c->hit_capacity == 0 && ensure_hits(c, (size_t)n * 32) != UPBP_OK) return UPBP_ERR_CUDA;
+            unsigned launches = 0;
+            size_t h2d = 0, d2h = 0;
+            unsigned long long found = 0;
+            const int rc = search_rounds(c, mode, n, launches, h2d, d2h, found, [&](unsigned long long total) {
+                k_debug_collect<<<1184, 128, 0, c->st>>>(c->d_hit_qb, total, t.counts, t.ids, ids_per_query);
+            });
+            if (rc != UPBP_OK) return rc;
+        }
+        UPBP_CK(cudaMemcpyAsync(counts, t.counts, n * sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
+        if (ids && id_bytes) UPBP_CK(cudaMemcpyAsync(ids, t.ids, id_bytes, cudaMemcpyDeviceToHost, c->st));
         UPBP_CK(cudaStreamSynchronize(c->st));
         return UPBP_OK;
     });

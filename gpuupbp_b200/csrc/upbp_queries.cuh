@@ -4,8 +4,12 @@
 // calls f for every photon or beam that passes the estimator's exact
 // predicate; the neighbour set is therefore defined by the predicate alone
 // (the reference's OptiX intersection programs apply the same predicates,
-// gpuupbp/kernel/pde/program_*.cu).  The estimators and the diagnostic
-// neighbour-set query both use these walkers.
+// gpuupbp/kernel/pde/program_*.cu).  Rendering uses points_in_radius_warp
+// (SURF, PP3D) and the packet searches of upbp_range_search.cuh, which share
+// the leaf tests here; the walkers of one query per lane (points_in_radius,
+// points_near_segment, beams_near_segment, beams_near_point) serve the
+// diagnostic neighbour-set query (upbp_debug_query), another route to the
+// same sets.
 #pragma once
 
 #include "upbp_paths.cuh"
@@ -35,11 +39,11 @@ UPBP_D void points_in_radius(const PointMap& map, float3 x, float r2, F&& f)
 
 // The same by a whole warp, one query per lane (`on` tells which lanes have
 // one): f as above, at most once a step, and step() by every lane after each
-// step of the walks.
+// step of the walks.  The caller counts what it merges.
 template <class F, class S>
 UPBP_D void points_in_radius_warp(bool on, const PointMap& map, float3 x, float r2, F&& f, S&& step)
 {
-    unsigned visits = 0, cand = 0, hits = 0;
+    unsigned visits = 0, cand = 0;
     bool ok = true;
     int stack[kStackDepth];
     int sp = 0;
@@ -65,10 +69,7 @@ UPBP_D void points_in_radius_warp(bool on, const PointMap& map, float3 x, float 
             const int first = leaf_first(node), cnt = leaf_count(node);
             const float4 pp = __ldg(&map.pos[first]);
             cand++;
-            if (pred_point_point(x, xyz(pp), r2)) {
-                hits++;
-                f(fbits(pp.w));
-            }
+            if (pred_point_point(x, xyz(pp), r2)) f(fbits(pp.w));
             if (cnt > 1)
                 node = leaf_link(first + 1, cnt - 1);
             else
@@ -80,7 +81,6 @@ UPBP_D void points_in_radius_warp(bool on, const PointMap& map, float3 x, float 
     if (!on) return;
     count_work(kCtrNodes, visits);
     count_work(kCtrPointCand, cand);
-    count_work(kCtrPointHit, hits);
     if (!ok) flag_status(kErrTraversalStack);
 }
 

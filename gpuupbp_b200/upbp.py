@@ -122,7 +122,7 @@ EXPORTS = ["upbp_parse_command_line", "upbp_scene_load_obj", "upbp_scene_load_pr
            "upbp_write_image", "upbp_get_stream", "upbp_last_error",
            "upbp_debug_photons", "upbp_debug_query", "upbp_debug_query_static", "upbp_get_device",
            "upbp_debug_mis_records", "upbp_guide_info", "upbp_guide_gradients", "upbp_run_batch",
-           "upbp_set_grid_limit", "upbp_debug_scene_bvh", "upbp_debug_beam_map", "upbp_save_checkpoint", "upbp_load_checkpoint"]
+           "upbp_set_grid_limit", "upbp_debug_scene_bvh", "upbp_debug_beam_map", "upbp_debug_search", "upbp_save_checkpoint", "upbp_load_checkpoint"]
 
 _libs = {}
 
@@ -167,6 +167,8 @@ def load_library(path: str = LIB_PATH):
     L.upbp_debug_scene_bvh.argtypes = [VP, ctypes.c_int, VP, ctypes.c_uint64, VP, ctypes.c_uint64,
                                        P(ctypes.c_uint32)]
     L.upbp_debug_beam_map.argtypes = [VP, VP]
+    L.upbp_debug_search.argtypes = [VP, ctypes.c_int, VP, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_float, VP, VP,
+                                    ctypes.c_uint32]
     L.upbp_save_checkpoint.argtypes = [VP, ctypes.c_char_p]
     L.upbp_load_checkpoint.argtypes = [VP, ctypes.c_char_p]
     _libs[path] = L
@@ -331,12 +333,21 @@ class Renderer:
         return out
 
     def query(self, kind: int, queries: np.ndarray, cap: int = 4096):
-        """Neighbour sets of the estimators' range queries (upbp_debug_query)."""
+        """Neighbour sets by a walk per query (upbp_debug_query)."""
         q = np.ascontiguousarray(queries, np.float32).reshape(-1, 8)
         counts = np.zeros(len(q), np.uint32)
         ids = np.zeros((len(q), cap), np.uint32)
         _check(self._L.upbp_debug_query(self._ctx, kind, q.ctypes.data, len(q), counts.ctypes.data,
                                                ids.ctypes.data, cap), "query")
+        return [ids[i, :min(int(c), cap)].copy() for i, c in enumerate(counts)], counts
+
+    def search(self, kind: int, queries: np.ndarray, unit_max: int = 0, spread: float = 0.0, cap: int = 4096):
+        """Neighbour sets of the searches that render (upbp_debug_search)."""
+        q = np.ascontiguousarray(queries, np.float32).reshape(-1, 8)
+        counts = np.zeros(len(q), np.uint32)
+        ids = np.zeros((len(q), cap), np.uint32)
+        _check(self._L.upbp_debug_search(self._ctx, kind, q.ctypes.data, len(q), unit_max, spread, counts.ctypes.data,
+                                         ids.ctypes.data, cap), "search", self._L)
         return [ids[i, :min(int(c), cap)].copy() for i, c in enumerate(counts)], counts
 
     def beam_map(self) -> dict:

@@ -316,8 +316,9 @@ int upbp_write_image(const char* path, const float* rgb, uint32_t width, uint32_
  * order; kind 2: beams as 8 floats (origin xyz, length, direction xyz,
  * light-path index bits).  *count receives the total; at most `capacity`
  * records are written.
- * upbp_debug_query: neighbour sets through the estimators' own range
- * queries for the last iteration's maps and radii.  Each query is 8 floats
+ * upbp_debug_query: neighbour sets of the last iteration's maps and radii
+ * by a walk per query through the maps' uncompressed nodes (the searches
+ * that render are upbp_debug_search).  Each query is 8 floats
  * (x y z dx dy dz tmin tmax).  kind 0 SURF and 1 PP3D (points within the
  * radius of x), 2 PB2D (medium photons along the segment), 3 BB1D (beams
  * near the segment), 4 BP2D (beams near x).  counts[i] = set size, ids =
@@ -335,6 +336,17 @@ int upbp_debug_scene_bvh(upbp_ctx* ctx, int real, float* nodes, uint64_t node_ca
                          uint64_t tri_capacity, uint32_t* count);
 int upbp_debug_query(upbp_ctx* ctx, int kind, const float* queries, uint32_t n, uint32_t* counts, uint32_t* ids,
                      uint32_t ids_per_query);
+/* upbp_debug_search: the same sets through the searches that render: the
+ * packet searches of PB2D, BB1D and BP2D (kinds 2-4) with their hit list and
+ * rounds, and the merging walk of SURF and PP3D (kinds 0-1).  The queries are
+ * searched in the order given (an iteration sorts its own); segment
+ * directions must be of unit length (UPBP_ERR_ARGS otherwise).  unit_max
+ * (a power of two up to 32) and group_spread set how kinds 2-4 share walks: at
+ * most so many queries a warp takes at once, and the largest extent of the
+ * start or end points of queries that share one (0: as in an iteration).  ids
+ * in no fixed order. */
+int upbp_debug_search(upbp_ctx* ctx, int kind, const float* queries, uint32_t n, uint32_t unit_max,
+                      float group_spread, uint32_t* counts, uint32_t* ids, uint32_t ids_per_query);
 /* upbp_debug_beam_map: the last iteration's beam map: its chunks (leaves),
  * and of its clustering the many-cluster passes, the final block's
  * iterations and the blocks of its launch (0 for the Morton-split LBVH). */

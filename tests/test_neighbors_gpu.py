@@ -1,7 +1,8 @@
-"""Photon neighbour sets of the five range queries equal a brute-force search
-with the same exact predicates, bit for bit (oracle/neighbors.py).  Queries
-are drawn around the stored photons so the sets are not empty, plus
-segments through the media."""
+"""Photon neighbour sets of the five range queries by a walk per query through
+the maps (upbp_debug_query) equal a brute-force search with the same exact
+predicates, bit for bit (oracle/neighbors.py).  The searches that render are
+compared in tests/test_neighbor_search_gpu.py.  Queries are drawn around the
+stored photons so the sets are not empty, plus segments through the media."""
 import numpy as np
 import pytest
 
