@@ -1,8 +1,8 @@
-"""The clustered beam map at the sizes where its kernels change shape: two
-chunks, less and more than a tile of 512 clusters, around the 1024 clusters
-one block finishes, several tiles.  Every size finds the pairs of the
-Morton-split LBVH (UPBP_BEAM_MAP=lbvh), and renders the same image up to the
-order of the float additions: 1e-4 as in tests/test_range_search_gpu.py."""
+"""The clustered beam map at the sizes where its kernels change shape: one
+chunk (no tree), two and three, around a tile of 512 clusters, around the
+1024 clusters one block finishes, several tiles.  Every size finds the pairs
+of the Morton-split LBVH (UPBP_BEAM_MAP=lbvh), and renders the same image up to
+the order of the float additions: 1e-4 as in tests/test_range_search_gpu.py."""
 import os
 
 import numpy as np
@@ -27,32 +27,59 @@ def _render(args, lbvh):
     return status, st, img
 
 
-# light paths; the chunks they give are asserted below to span the sizes
-@pytest.mark.parametrize("paths,radius", [(3, -0.2), (5, -0.02), (60, -0.05), (120, -0.02), (330, -0.02), (420, -0.02),
-                                          (900, -0.02), (4000, -0.02)])
-def test_clustered_map_equals_lbvh(scene_dir, paths, radius):
-    path = scenes.write_workload("box_medium", scene_dir, tiny=True)
-    args = ["-s", "-1", path, "-a", "upbp_bb1d+bp2d", "-l", "8", "-r", "33x29", "-pcpi", str(paths),
-            "-r_initial", str(radius)]
+def _compare(args):
     s0, a, img0 = _render(args, False)
     s1, b, img1 = _render(args, True)
     assert s0 == s1 and a["beam_chunks"] == b["beam_chunks"] and b["beam_map_passes"] == 0
     assert (a["beam_map_passes"] > 0) == (a["beam_chunks"] > 1)
     for k in ("bb1d_query", "bp2d_query"):
-        assert a["work"][k]["beam_hit"] == b["work"][k]["beam_hit"], k
+        assert a["work"][k]["beam_hit"] == b["work"][k]["beam_hit"] > 0, k
     assert np.allclose(img0, img1, rtol=1e-4, atol=1e-7)
+    return a["beam_chunks"]
 
 
-def test_sizes_span_the_tiles(scene_dir):
-    """The light paths above give fewer than 512, about 1024 and several
-    thousand chunks."""
+# light paths and radii
+@pytest.mark.parametrize("paths,radius", [(5, -0.02), (60, -0.05), (420, -0.02), (900, -0.02), (4000, -0.02)])
+def test_clustered_map_equals_lbvh(scene_dir, paths, radius):
     path = scenes.write_workload("box_medium", scene_dir, tiny=True)
-    got = []
-    for paths in (60, 330, 4000):
-        _, st, _ = _render(["-s", "-1", path, "-a", "upbp_bb1d+bp2d", "-l", "8", "-r", "33x29", "-pcpi", str(paths),
-                            "-r_initial", "-0.02"], False)
-        got.append(st["beam_chunks"])
-    assert 0 < got[0] < 512 and 512 < got[1] < 2048 and got[2] > 4096
+    chunks = _compare(["-s", "-1", path, "-a", "upbp_bb1d+bp2d", "-l", "8", "-r", "33x29", "-pcpi", str(paths),
+                       "-r_initial", str(radius)])
+    assert chunks > 4096 or paths < 4000
+
+
+def _chunks(lengths, radius):
+    """Chunks of beams of these lengths: one for every six radii, at most 64."""
+    step = np.float32(6.0) * np.float32(radius)
+    return int(np.maximum(1, np.minimum(np.ceil(lengths / step), 64)).sum())
+
+
+@pytest.mark.parametrize("paths,chunks", [(1, 2), (1, 3), (200, 511), (200, 512), (200, 513), (300, 1023), (300, 1024),
+                                          (300, 1025)])
+def test_exact_sizes(scene_dir, paths, chunks):
+    """The radius that gives exactly this many chunks: their number falls with
+    the radius, a beam at a time."""
+    from gpuupbp_b200 import upbp
+    path = scenes.write_workload("box_medium", scene_dir, tiny=True)
+    args = ["-s", "-1", path, "-a", "upbp_bb1d+bp2d", "-l", "8", "-r", "33x29", "-pcpi", str(paths), "-r_initial"]
+    r = upbp.Renderer(args + ["-0.02"])
+    r.run_iteration(1)  # the light paths depend on the iteration alone, not on the radius
+    lengths = r.photons(2)[:, 3].copy()
+    r.close()
+    assert 0 < len(lengths) <= chunks
+    lo, hi = np.float32(1e-6).view(np.int32), np.float32(10.0).view(np.int32)  # the order of floats is that of their bits
+    while hi - lo > 1:
+        mid = (int(lo) + int(hi)) // 2
+        lo, hi = (mid, hi) if _chunks(lengths, np.int32(mid).view(np.float32)) >= chunks else (lo, mid)
+    radius = np.int32(lo).view(np.float32)
+    assert _chunks(lengths, radius) == chunks
+    assert _compare(args + ["%.9g" % radius]) == chunks
+    r = upbp.Renderer(args + ["%.9g" % radius])
+    r.run_iteration(1)
+    info = r.beam_map()
+    r.close()
+    # many-cluster passes from 1025 clusters on, one block of 512 clusters a tile
+    assert info["chunks"] == chunks and (info["passes"] > 0) == (chunks > 1024)
+    assert info["blocks"] == -(-chunks // 512) and info["tail_iterations"] > 0
 
 
 def _blocks(scene_dir, env, limit):

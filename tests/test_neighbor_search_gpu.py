@@ -194,6 +194,33 @@ def test_near_perpendicular_bb1d(scene_dir):
     r.close()
 
 
+@pytest.mark.parametrize("iteration,leaves", [(0, (1, 0)), (1, (2, 1)), (4, (0, 0))])
+def test_smallest_maps(scene_dir, iteration, leaves):
+    """A beam map of one chunk and of two, a medium photon map of one, empty
+    maps: one light path at a radius of a fifth of the scene's."""
+    from gpuupbp_b200 import upbp
+    path = scenes.write_workload("box_medium", scene_dir, tiny=True)
+    r = upbp.Renderer(["-s", "-1", path, "-a", ALL6, "-l", "8", "-r", "33x29", "-pcpi", "1", "-r_initial", "-0.2"])
+    r.run_iteration(iteration)
+    rb1, rb2, rpb, rpp, rsu, _ = r.stats()["radius"]
+    med, beams = r.photons(1), r.photons(2)
+    assert (len(beams), len(med)) == leaves and r.beam_map()["chunks"] == leaves[0]
+    slots = med[:, 3].view(np.uint32)
+    rng = np.random.default_rng(47)
+    n = 77
+    centres = rng.uniform(-0.5, 0.5, (n, 3))
+    if len(beams):
+        centres = beams[rng.integers(0, len(beams), n), :3] + rng.normal(size=(n, 3)) * 0.1
+    q, x = _segments(rng, centres, 0.5), _points(centres)
+    sizes = [_check(r, 2, q, lambda qq: slots[neighbors.points_near_segment(med, qq, np.float32(rpb) ** 2)], rpb),
+             _check(r, 3, q, lambda qq: neighbors.beams_near_segment(beams, qq, np.float32(rb1) ** 2), rb1,
+                    ignore=lambda qq, i: _beam_pair_ill_posed(qq, beams[i], rb1)),
+             _check(r, 4, x, lambda qq: neighbors.beams_near_point(beams, qq[:3], np.float32(rb2) ** 2), rb2),
+             _check(r, 1, x, lambda qq: slots[neighbors.points_in_radius(med, qq[:3], np.float32(rpp) ** 2)], rpp)]
+    assert [bool(s.sum()) for s in sizes[:3]] == [leaves[1] > 0, leaves[0] > 0, leaves[0] > 0]
+    r.close()
+
+
 def test_short_hit_list(scene_dir):
     """A list that holds a few queries' pairs: rounds, repeated rounds, empty
     slots between the hits of a round."""

@@ -23,7 +23,10 @@ TECH = "upbp_bpt+surf+pp3d+pb2d+bb1d+bp2d"
 
 
 # one query and a remainder of a unit; one warp's worth and one more; a few
-# hundred queries; a one-beam map has no inner node (the last case: few light paths)
+# hundred queries; a beam map of one chunk, which has no inner node (ONE_LEAF)
+ONE_LEAF = ["-pcpi", "1", "-r_initial", "-0.2"]
+
+
 @pytest.mark.parametrize("workload,res,extra", [
     ("box_medium", "2x1", []),
     ("box_medium", "8x4", []),
@@ -33,11 +36,12 @@ TECH = "upbp_bpt+surf+pp3d+pb2d+bb1d+bp2d"
     ("dense_beams", "41x23", ["-r_initial_bb1d", "-0.004", "-r_initial_bp2d", "-0.004", "-pbc", "300"]),
     ("media_field", "53x31", ["-pbt", "S"]),
     ("box_medium", "33x31", ["-pcpi", "3"]),
+    ("box_medium", "33x31", ONE_LEAF),
 ])
 def test_pairs_do_not_depend_on_the_split(scene_dir, workload, res, extra):
     from gpuupbp_b200 import upbp
     path = scenes.write_workload(workload, scene_dir, tiny=True)
-    radius = [] if workload in ("dense_beams", "media_field") else ["-r_initial", "-0.02"]
+    radius = [] if workload in ("dense_beams", "media_field") or "-r_initial" in extra else ["-r_initial", "-0.02"]
     r = upbp.Renderer(["-s", "-1", path, "-a", TECH, "-l", "9", "-r", res] + radius + extra)
     got = []
     for limit in (0, 1, 3):
@@ -47,6 +51,8 @@ def test_pairs_do_not_depend_on_the_split(scene_dir, workload, res, extra):
         got.append((status, r.iteration_image(), {k: (w["beam_hit"], w["point_hit"]) for k, w in st["work"].items()},
                     st["light_beams"]))
     r.close()
+    if extra == ONE_LEAF:
+        assert st["beam_chunks"] == 1 and st["work"]["bb1d_query"]["beam_hit"] > 0
     for status, img, hits, beams in got[1:]:
         assert status == got[0][0] and beams == got[0][3]
         assert hits == got[0][2]
