@@ -389,7 +389,6 @@ UPBP_D bool closest_hit(bool on, const TriView& tv, float3 o, float3 d, float tm
 
 // The stack of a warp's all_hits: (link, lane that owns the ray) entries.
 constexpr int kAllHitsStack = 448;
-constexpr int kRayWarps = 4;  // warps of the blocks that cast rays
 // Triangles few enough to test one after the other, the lanes together (the
 // boxes of the predefined scenes: camera extend 0.34 -> 0.27 ms at 512x512); a
 // sphere of 1280 triangles is faster shared.
@@ -398,7 +397,7 @@ struct AllHitsStack {
     int link[kAllHitsStack];
     unsigned char owner[kAllHitsStack];
 };
-__shared__ AllHitsStack s_all_hits[kRayWarps];
+__shared__ AllHitsStack s_all_hits[kPassWarps];
 
 // Every triangle hit with t in [tmin, tmax], in no order but each with its
 // leaf position (h.u, as an int; ascending positions are the order of a

@@ -682,7 +682,6 @@ UPBP_D float3 eval_range_hit(uint2 qb, unsigned& px, FQ&& fq, FN&& fn)
 // addresses, which kept the L1 busy), then every lane takes its own record
 // from shared memory (rows padded to 144 bytes, so the eight lanes of a
 // quarter-warp read different banks).  rec is this lane's record.
-constexpr int kEvalWarps = 4;
 UPBP_D void gather_records(const float4* rec, float4 (&out)[8], float4 (*s)[9], unsigned lane)
 {
     __syncwarp();
@@ -701,7 +700,8 @@ UPBP_D void gather_records(const float4* rec, float4 (&out)[8], float4 (*s)[9], 
 // The query records of a warp's 32 hits: consecutive hits mostly share their
 // query (the search finds a query's pairs side by side), so a record is
 // loaded once per run of equal queries, four records at a time, and its
-// lanes read the run's row.  `run` is the lane's run, `runs` their number.
+// lanes read the run's row.  `run` is the lane's run, `heads` has a bit at the
+// first lane of each.
 UPBP_D void gather_runs(const float4* rec, unsigned run, unsigned heads, float4 (&out)[8], float4 (*s)[9],
                         const float4** first, unsigned lane)
 {
@@ -720,13 +720,13 @@ UPBP_D void gather_runs(const float4* rec, unsigned run, unsigned heads, float4 
 // kGuided: a learned-proposal table is in use (the unguided instantiation,
 // the common case, contains none of the proposal's code).
 template <int kMode, bool kGuided>
-__global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 7) range_eval_kernel(int slot)
 {
     using M = RangeMode<kMode>;
     begin_kernel(M::kern, slot);
     const DeviceParams& p = c_params;
-    __shared__ float4 s_rec[kEvalWarps][32][9];
-    __shared__ const float4* s_first[kEvalWarps][32];
+    __shared__ float4 s_rec[kPassWarps][32][9];
+    __shared__ const float4* s_first[kPassWarps][32];
     float4(*s)[9] = s_rec[threadIdx.x >> 5];
     const float4** first = s_first[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
@@ -785,13 +785,12 @@ __global__ void __launch_bounds__(128, 7) range_eval_kernel(int slot)
 // end: evaluated where they are found, about 60 merges of a warp at almost as
 // many different steps each ran on one or two lanes.
 constexpr unsigned kPendingMerges = 8;
-constexpr int kMergeThreads = 128;  // of the blocks that merge points
 
 // merge(slot), on the query's lane, for every photon within the radius of x.
 template <class F>
 UPBP_D void merge_points(bool on, const PointMap& map, float3 x, float r2, F&& merge)
 {
-    __shared__ unsigned s_found[kPendingMerges][kMergeThreads];
+    __shared__ unsigned s_found[kPendingMerges][kPassThreads];
     unsigned found = 0, merged = 0;
     auto flush = [&]() {
         for (unsigned i = 0; i < found; i++) merge(s_found[i][threadIdx.x]);
@@ -808,7 +807,7 @@ UPBP_D void merge_points(bool on, const PointMap& map, float3 x, float r2, F&& m
 }
 
 template <bool medium, bool kGuided>
-__global__ void __launch_bounds__(kMergeThreads, 5) point_merge_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 5) point_merge_kernel(int slot)
 {
     begin_kernel(medium ? kKernPp3d : kKernSurf, slot);
     const DeviceParams& p = c_params;
@@ -1095,7 +1094,7 @@ UPBP_D void camera_path_end(const CameraLane& c)
 // the next pixel from a global counter instead of idling until the longest
 // path of its warp is done.  Each pixel's random stream depends on the pixel
 // alone, so the assignment of pixels to lanes does not change any path.
-__global__ void __launch_bounds__(128, 8) camera_pass_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 8) camera_pass_kernel(int slot)
 {
     begin_kernel(kKernCameraExtend, slot);
     const DeviceParams& p = c_params;
@@ -1137,7 +1136,7 @@ __global__ void __launch_bounds__(128, 8) camera_pass_kernel(int slot)
 // Deferred NEE: one light sample per thread -- occlusion ray through the
 // media, MIS weight, throughput.  The contribution is kept per sample until
 // k_resolve_camera knows whether an earlier step of the path failed.
-__global__ void __launch_bounds__(128, 8) nee_connect_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 8) nee_connect_kernel(int slot)
 {
     begin_kernel(kKernNee, slot);
     const DeviceParams& p = c_params;
@@ -1198,7 +1197,7 @@ __global__ void __launch_bounds__(128, 8) nee_connect_kernel(int slot)
 // Deferred BPT: one (camera vertex, light vertex) pair per thread -- the
 // path-length and media checks of the connection loop, then the connection
 // with its occlusion ray; the contribution is kept per pair like NEE's.
-__global__ void __launch_bounds__(128, 8) bpt_connect_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 8) bpt_connect_kernel(int slot)
 {
     begin_kernel(kKernBpt, slot);
     const DeviceParams& p = c_params;

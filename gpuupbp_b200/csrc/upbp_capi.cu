@@ -241,7 +241,7 @@ __global__ void k_debug_collect(const uint2* hits, unsigned long long total, uns
 
 // Neighbour sets through the merging walk of SURF and PP3D.
 template <bool medium>
-__global__ void __launch_bounds__(kMergeThreads) k_debug_merge(int slot, const float* q, unsigned n, unsigned* counts,
+__global__ void __launch_bounds__(kPassThreads) k_debug_merge(int slot, const float* q, unsigned n, unsigned* counts,
                                                                unsigned* ids, unsigned cap)
 {
     begin_kernel(kKernDebug, slot);
@@ -378,7 +378,6 @@ struct upbp_ctx {
 
 namespace {
 
-// Blocks of a launch under the context's grid limit (at least one).
 // Borrows the largest idle hit list of the context's device for one call
 // and returns it (after the call's kernels are done) at the end.
 class HitLease {
@@ -390,6 +389,7 @@ class HitLease {
     upbp_ctx* c_;
 };
 
+// Blocks of a launch under the context's grid limit (at least one).
 unsigned cap_grid(const upbp_ctx* c, unsigned blocks)
 {
     return c->grid_limit ? std::max(1u, std::min(blocks, c->grid_limit)) : blocks;
@@ -1029,7 +1029,7 @@ void range_search_split(DeviceParams& P, int mode)
 // hits wait for it, and used whole.
 unsigned hit_reserve_limit(unsigned capacity, unsigned blocks)
 {
-    return std::max(32u, std::min(512u, capacity / (8u * kSearchWarps * blocks) & ~31u));
+    return std::max(32u, std::min(512u, capacity / (8u * kPassWarps * blocks) & ~31u));
 }
 
 // Largest range-query hit list (8 bytes per entry, 34 GB, allocated only
@@ -1102,9 +1102,9 @@ int search_rounds(upbp_ctx* c, int mode, unsigned nq, unsigned& launches, size_t
         h2d += sizeof(P);
         UPBP_CK(upload_params(c));
         switch (mode) {
-        case kModePb2d: PK(c).range_search[kModePb2d]<<<g, 128, 0, c->st>>>(c->slot); break;
-        case kModeBb1d: PK(c).range_search[kModeBb1d]<<<g, 128, 0, c->st>>>(c->slot); break;
-        default: PK(c).range_search[kModeBp2d]<<<g, 128, 0, c->st>>>(c->slot); break;
+        case kModePb2d: PK(c).range_search[kModePb2d]<<<g, kPassThreads, 0, c->st>>>(c->slot); break;
+        case kModeBb1d: PK(c).range_search[kModeBb1d]<<<g, kPassThreads, 0, c->st>>>(c->slot); break;
+        default: PK(c).range_search[kModeBp2d]<<<g, kPassThreads, 0, c->st>>>(c->slot); break;
         }
         launches++;
         UPBP_CK(cudaGetLastError());
@@ -1401,19 +1401,19 @@ extern "C" int upbp_create(const upbp_scene_desc* s, const upbp_config* cfg, upb
                                                (const void*)range_search_kernel<kModeBb1d>,
                                                (const void*)range_search_kernel<kModeBp2d>};
             for (int m = 0; m < kRangeModes; m++) {
-                UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, search[m], 128, 0));
+                UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, search[m], kPassThreads, 0));
                 c->search_grid[m] = std::max(1, sms * std::max(1, per_sm));
             }
             const void* eval[kRangeModes] = {(const void*)range_eval_kernel<kModePb2d, false>,
                                              (const void*)range_eval_kernel<kModeBb1d, false>,
                                              (const void*)range_eval_kernel<kModeBp2d, false>};
             for (int m = 0; m < kRangeModes; m++) {
-                UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval[m], 128, 0));
+                UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval[m], kPassThreads, 0));
                 c->eval_grid[m] = std::max(1, sms * std::max(1, per_sm));
             }
-            UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, camera_pass_kernel, 128, 0));
+            UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, camera_pass_kernel, kPassThreads, 0));
             c->camera_grid = std::max(1, sms * std::max(1, per_sm));
-            UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, light_pass_kernel, 128, 0));
+            UPBP_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, light_pass_kernel, kPassThreads, 0));
             c->light_grid = std::max(1, sms * std::max(1, per_sm));
         }
         c->seg_capacity = std::max(1024u, 4 * P.screen_pixel_count);
@@ -1632,7 +1632,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             h2d += sizeof(P);
             UPBP_CK(upload_params(c));
             if (L > 0) {
-                PK(c).light_pass<<<cap_grid(c, std::min<unsigned>(c->light_grid, (L + 127) / 128)), 128, 0, c->st>>>(
+                PK(c).light_pass<<<cap_grid(c, std::min<unsigned>(c->light_grid, (L + kPassThreads - 1) / kPassThreads)), kPassThreads, 0, c->st>>>(
                     c->slot);
                 launches++;
             }
@@ -1782,8 +1782,8 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 UPBP_CK(upload_params(c));
                     UPBP_CK(cudaMemsetAsync(c->d_work + (size_t)kKernCameraExtend * kCtrCount, 0,
                                         kCtrCount * sizeof(unsigned long long), c->st));
-                PK(c).camera_pass<<<cap_grid(c, std::min<unsigned>(c->camera_grid, (P.screen_pixel_count + 127) / 128)),
-                                     128, 0, c->st>>>(c->slot);
+                PK(c).camera_pass<<<cap_grid(c, std::min<unsigned>(c->camera_grid, (P.screen_pixel_count + kPassThreads - 1) / kPassThreads)),
+                                     kPassThreads, 0, c->st>>>(c->slot);
                 launches++;
                 UPBP_CK(cudaGetLastError());
                 d2h += 6 * sizeof(unsigned);
@@ -1845,7 +1845,7 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
             }
         }
         UPBP_CK(cudaEventRecord(ev[3], c->st));
-        auto grid_for = [c](unsigned n) { return cap_grid(c, std::max(1u, std::min((n + 127) / 128, 148u * 64u))); };
+        auto grid_for = [c](unsigned n) { return cap_grid(c, std::max(1u, std::min((n + kPassThreads - 1) / kPassThreads, 148u * 64u))); };
         // deferred NEE and BPT connections, then the colours of every camera path
         // whose steps all succeeded (the query kernels below check the same)
         const unsigned nnee = P.trace_camera_paths ? std::min(c->h_qcount[4], c->nee_capacity) : 0;
@@ -1853,12 +1853,12 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
         if (P.trace_camera_paths)
             UPBP_CK(cudaMemsetAsync(c->d_path_err, 0xff, P.screen_pixel_count * sizeof(unsigned), c->st));
         if (nnee > 0) {
-            PK(c).nee_connect<<<grid_for(nnee), 128, 0, c->st>>>(c->slot);
+            PK(c).nee_connect<<<grid_for(nnee), kPassThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         UPBP_CK(cudaEventRecord(ev[4], c->st));
         if (nbpt > 0) {
-            PK(c).bpt_connect<<<grid_for(nbpt), 128, 0, c->st>>>(c->slot);
+            PK(c).bpt_connect<<<grid_for(nbpt), kPassThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         if (P.trace_camera_paths) {
@@ -1903,20 +1903,20 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
                 // wave of resident blocks swept the whole list and read
                 // the records again
                 const unsigned g2 = cap_grid(
-                    c, std::max(1u, std::min<unsigned>((unsigned)((total + 127) / 128), (unsigned)c->eval_grid[mode])));
+                    c, std::max(1u, std::min<unsigned>((unsigned)((total + kPassThreads - 1) / kPassThreads), (unsigned)c->eval_grid[mode])));
                 const bool gd = P.guide.entries != nullptr;
                 switch (mode) {
                 case kModePb2d:
-                    if (gd) PK(c).range_eval[kModePb2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                    else PK(c).range_eval[kModePb2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    if (gd) PK(c).range_eval[kModePb2d][1]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModePb2d][0]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
                     break;
                 case kModeBb1d:
-                    if (gd) PK(c).range_eval[kModeBb1d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                    else PK(c).range_eval[kModeBb1d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    if (gd) PK(c).range_eval[kModeBb1d][1]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModeBb1d][0]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
                     break;
                 default:
-                    if (gd) PK(c).range_eval[kModeBp2d][1]<<<g2, 128, 0, c->st>>>(c->slot);
-                    else PK(c).range_eval[kModeBp2d][0]<<<g2, 128, 0, c->st>>>(c->slot);
+                    if (gd) PK(c).range_eval[kModeBp2d][1]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
+                    else PK(c).range_eval[kModeBp2d][0]<<<g2, kPassThreads, 0, c->st>>>(c->slot);
                     break;
                 }
             });
@@ -1928,14 +1928,14 @@ extern "C" int upbp_run_iteration(upbp_ctx* c, int iteration)
         };
         UPBP_CK(cudaEventRecord(ev[6], c->st));
         if (run_surf) {
-            if (P.guide.entries) PK(c).point_merge[0][1]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
-            else PK(c).point_merge[0][0]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
+            if (P.guide.entries) PK(c).point_merge[0][1]<<<grid_for(npt), kPassThreads, 0, c->st>>>(c->slot);
+            else PK(c).point_merge[0][0]<<<grid_for(npt), kPassThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         UPBP_CK(cudaEventRecord(ev[7], c->st));
         if (run_pp3d) {
-            if (P.guide.entries) PK(c).point_merge[1][1]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
-            else PK(c).point_merge[1][0]<<<grid_for(npt), kMergeThreads, 0, c->st>>>(c->slot);
+            if (P.guide.entries) PK(c).point_merge[1][1]<<<grid_for(npt), kPassThreads, 0, c->st>>>(c->slot);
+            else PK(c).point_merge[1][0]<<<grid_for(npt), kPassThreads, 0, c->st>>>(c->slot);
             launches++;
         }
         UPBP_CK(cudaEventRecord(ev[8], c->st));
@@ -2277,9 +2277,9 @@ extern "C" int upbp_debug_search(upbp_ctx* c, int kind, const float* queries, ui
         SlotLease lease(c->dev, c->slot, c->st);
         if (kind < 2) {
             UPBP_CK(upload_params(c));
-            const unsigned g = (n + kMergeThreads - 1) / kMergeThreads;
-            if (kind == 0) k_debug_merge<false><<<g, kMergeThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
-            else k_debug_merge<true><<<g, kMergeThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
+            const unsigned g = (n + kPassThreads - 1) / kPassThreads;
+            if (kind == 0) k_debug_merge<false><<<g, kPassThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
+            else k_debug_merge<true><<<g, kPassThreads, 0, c->st>>>(c->slot, t.q, n, t.counts, t.ids, ids_per_query);
             UPBP_CK(cudaGetLastError());
         } else if ((kind == 2 ? P.med_map.bvh.count : P.beam_map.bvh.count) > 0) {
             const int mode = kind == 2 ? kModePb2d : kind == 3 ? kModeBb1d : kModeBp2d;

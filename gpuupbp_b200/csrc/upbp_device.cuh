@@ -474,6 +474,11 @@ UPBP_D void begin_kernel(int kind, int slot)
 // c_params.work): the running kernel's set.
 UPBP_D unsigned long long* c_work_ptr() { return c_params.work + (size_t)s_kernel_kind * kCtrCount; }
 
+// Threads of a block of the passes, connections, searches, evaluations and
+// point merges: their shared memory holds a part for each of its warps.
+constexpr int kPassThreads = 128;
+constexpr int kPassWarps = kPassThreads / 32;
+
 // Kernel kinds of an iteration, for work counters and timing.  The
 // diagnostic neighbour queries count into a row of their own after the
 // iteration's rows (kKernDebug), so they never change an iteration's figures.

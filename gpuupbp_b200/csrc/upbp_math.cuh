@@ -43,6 +43,8 @@ UPBP_HD float max_component(float3 a) { return fmaxf(a.x, fmaxf(a.y, a.z)); }
 UPBP_HD float component(float3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
 UPBP_HD float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
+UPBP_D float3 min3f(float3 a, float3 b) { return make_float3(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)); }
+UPBP_D float3 max3f(float3 a, float3 b) { return make_float3(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)); }
 UPBP_HD bool is_black_or_negative(float3 a) { return a.x <= 0.f && a.y <= 0.f && a.z <= 0.f; }
 UPBP_HD bool is_positive(float a) { return a > 1e-20f; }
 UPBP_HD bool is_positive(float3 a) { return is_positive(a.x) && is_positive(a.y) && is_positive(a.z); }

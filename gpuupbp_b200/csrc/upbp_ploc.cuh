@@ -73,8 +73,6 @@ UPBP_D float ploc_area(float3 lo, float3 hi)
     return dx * dy + dy * dz + dz * dx;
 }
 
-UPBP_D float3 min3f(float3 a, float3 b) { return make_float3(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)); }
-UPBP_D float3 max3f(float3 a, float3 b) { return make_float3(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)); }
 
 // Leaves in Morton order (vals: chunk per Morton position), which is also the
 // leaf order of a tree that does not get laid out.

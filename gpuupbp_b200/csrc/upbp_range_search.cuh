@@ -34,7 +34,6 @@
 
 namespace upbp {
 
-constexpr int kSearchWarps = 4;
 constexpr int kPacketStack = 384;   // stack of a warp: node | group << kLeafShift
 constexpr int kPacketLeaves = 160;  // < 32 waiting + 128 of a step
 
@@ -59,8 +58,6 @@ struct PacketBox {
     float3 alo, ahi, blo, bhi;
 };
 
-UPBP_D float3 min3(float3 a, float3 b) { return make_float3(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)); }
-UPBP_D float3 max3(float3 a, float3 b) { return make_float3(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)); }
 UPBP_D float3 shfl3_xor(float3 a, int m)
 {
     return make_float3(__shfl_xor_sync(~0u, a.x, m), __shfl_xor_sync(~0u, a.y, m), __shfl_xor_sync(~0u, a.z, m));
@@ -369,12 +366,12 @@ UPBP_D void packet_walk(SearchWarp& w, PacketState& s, unsigned lane, const QNod
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(128, 7) range_search_kernel(int slot)
+__global__ void __launch_bounds__(kPassThreads, 7) range_search_kernel(int slot)
 {
     using M = RangeMode<kMode>;
     begin_kernel(M::kern, slot);
     const DeviceParams& p = c_params;
-    __shared__ SearchWarp s_warp[kSearchWarps];
+    __shared__ SearchWarp s_warp[kPassWarps];
     SearchWarp& w = s_warp[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31;
     // this round's range of the processing order, within the queue
@@ -383,7 +380,7 @@ __global__ void __launch_bounds__(128, 7) range_search_kernel(int slot)
     // Queries a warp takes at once, a power of two: an even share of the
     // queries left, split units_per_warp ways so that the warps finish
     // together, and no more than unit_max (range_search_split).
-    const unsigned share = gridDim.x * kSearchWarps * p.units_per_warp;
+    const unsigned share = gridDim.x * kPassWarps * p.units_per_warp;
     auto next_unit = [&](unsigned left) {
         const unsigned u = left / share;
         return u >= p.unit_max ? p.unit_max : u <= 1u ? 1u : 1u << (31 - __clz(u));
@@ -473,11 +470,11 @@ __global__ void __launch_bounds__(128, 7) range_search_kernel(int slot)
             PacketBox b = box;
             for (int k = 0; (1u << k) < take; k++) {
                 const int x = 1 << k;
-                b.alo = min3(b.alo, shfl3_xor(b.alo, x));
-                b.ahi = max3(b.ahi, shfl3_xor(b.ahi, x));
+                b.alo = min3f(b.alo, shfl3_xor(b.alo, x));
+                b.ahi = max3f(b.ahi, shfl3_xor(b.ahi, x));
                 if constexpr (M::seg) {
-                    b.blo = min3(b.blo, shfl3_xor(b.blo, x));
-                    b.bhi = max3(b.bhi, shfl3_xor(b.bhi, x));
+                    b.blo = min3f(b.blo, shfl3_xor(b.blo, x));
+                    b.bhi = max3f(b.bhi, shfl3_xor(b.bhi, x));
                 }
                 float spread = max_component(b.ahi - b.alo);
                 if constexpr (M::seg) spread = fmaxf(spread, max_component(b.bhi - b.blo));
