@@ -164,14 +164,22 @@ class ClockSampler:
 # Algorithmic bytes of the camera-pass kernel per unit of counted work
 # (record sizes of this build's layouts): BVH node 64 B (two child boxes +
 # links), triangle 48 B (v0, e1, e2), per ray the hit's normals + record 72 B,
-# photon point 16 B, accepted photon's vertex record 128 B, beam chunk 48 B,
-# accepted beam record 128 B, BPT light-vertex record 128 B; plus 24 B of
-# framebuffer read-modify-write per pixel.
-BYTES_PER_WORK = {"nodes": 64, "tris": 48, "rays": 72, "point_cand": 16, "point_hit": 128, "beam_cand": 48,
+# photon point 16 B, accepted photon's vertex record 128 B, beam chunk 40 B (its
+# 8 B leaf and the beam's line), accepted beam record 128 B, BPT light-vertex
+# record 128 B; plus 24 B of framebuffer read-modify-write per pixel.
+# These are bytes the kernels ask for, from whatever level of the memory holds
+# them (L1 and L2 serve most of the range searches' and merges'): a rate above
+# the DRAM's is no error, and the figures of builds that count other units of
+# work (nodes a walk per query, two-wide nodes) don't compare.
+BYTES_PER_WORK = {"nodes": 64, "tris": 48, "rays": 72, "point_cand": 16, "point_hit": 128, "beam_cand": 40,
                   "beam_hit": 128, "vertex_loads": 128}
-# The PB2D, BB1D and BP2D searches count 32 bytes a node test (they read the
-# maps' 48-byte four-wide nodes, shared by the queries of a group).
+# The PB2D, BB1D and BP2D searches test the maps' 48-byte four-wide nodes,
+# once for a group of queries.  Of BB1D the counted candidates are the pairs left
+# for the exact test: the leaves of the conservative one are not counted.
 COMPRESSED_NODE_KERNELS = ("pb2d_query", "bb1d_query", "bp2d_query")
+COMPRESSED_NODE_BYTES = 48
+# What bounds a kernel where it isn't DRAM, from the counters in profiles/.
+BOUND_BY = {"bb1d_query": "issue and the L1 data pipe (profiles/bb1d_query_media_field.md)"}
 
 
 def algorithmic_bytes(work: dict, extra: float = 0.0, node_bytes: int = 64) -> float:
@@ -208,7 +216,7 @@ def kernel_rooflines(st: dict, pixels: int) -> dict:
     out = {}
     for k, w in st["work"].items():
         t = ms[k] / n
-        b = algorithmic_bytes(w, extra[k], 32 if k in COMPRESSED_NODE_KERNELS else 64)
+        b = algorithmic_bytes(w, extra[k], COMPRESSED_NODE_BYTES if k in COMPRESSED_NODE_KERNELS else 64)
         out[k] = {"ms": t, "bytes": b, "gbs": (b / (t * 1e-3) / 1e9) if t > 0 else 0.0}
     return out
 
@@ -365,7 +373,8 @@ def run_b200(args) -> dict | None:
         "gpu_launches": int(st["kernel_launches"]) * args.steps,
         "roofline": {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src,
-                     "traffic": traffic, "algorithmic_bytes_per_launch": b_top, "launch_ms": top_ms},
+                     "traffic": traffic, "algorithmic_bytes_per_launch": b_top, "launch_ms": top_ms,
+                     "bound_by": BOUND_BY.get(top, "see profiles/")},
         "iteration_roofline": iteration_roofline,
         "kernels": kernels,
         "clocks": clk.summary(window[0], window[-1]),

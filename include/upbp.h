@@ -218,7 +218,13 @@ typedef struct upbp_stats {
     /* Work counters of the last iteration, light pass then camera pass, in
      * the order: BVH node visits, triangle tests, rays cast, photon-point
      * candidates, accepted point merges, beam-chunk candidates, accepted beam
-     * merges, light-vertex records read by BPT connections. */
+     * merges, light-vertex records read by BPT connections.  The range
+     * searches (PB2D, BB1D, BP2D) walk for a group of queries at a time:
+     * their node visits are tests of a four-wide node against the bound of a
+     * group; their candidates are pairs of a leaf that a group reached with
+     * each of its queries (PB2D, BP2D), or those of these pairs that a
+     * conservative test leaves for the exact one (BB1D).  Counts of builds
+     * that walked per query, or two-wide nodes, are larger for the same work. */
     uint64_t work_light[8];
     uint64_t work_camera[8];
     uint32_t beam_chunks;         /* leaves of the last beam map */

@@ -1,5 +1,5 @@
 """bench.py's host-side arithmetic on synthetic counters: per-kernel
-algorithmic bytes (32-byte nodes for the range searches), the whole-iteration
+algorithmic bytes (48-byte nodes for the range searches), the whole-iteration
 roofline's record sizes, and the clock sampler's timed window."""
 import datetime
 import os
@@ -24,7 +24,7 @@ def fake_stats():
 def test_kernel_rooflines_use_compressed_node_bytes():
     k = bench.kernel_rooflines(fake_stats(), pixels=100)
     bb = k["bb1d_query"]
-    expect = 1000 * 32 + 100 * 48 + 10 * 128 + bench.SEG_RECORD * 7 + bench.HIT_RECORD * 2 * 10
+    expect = 1000 * 48 + 100 * 40 + 10 * 128 + bench.SEG_RECORD * 7 + bench.HIT_RECORD * 2 * 10
     assert bb["bytes"] == expect and bb["ms"] == 1.0
     assert k["light_pass"]["bytes"] == 500 * 64 + 50 * 48 + 5 * 72
 
