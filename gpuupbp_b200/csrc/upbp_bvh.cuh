@@ -389,9 +389,11 @@ UPBP_D bool closest_hit(bool on, const TriView& tv, float3 o, float3 d, float tm
 
 // The stack of a warp's all_hits: (link, lane that owns the ray) entries.
 constexpr int kAllHitsStack = 448;
-// Triangles few enough to test one after the other, the lanes together (the
-// boxes of the predefined scenes: camera extend 0.34 -> 0.27 ms at 512x512); a
-// sphere of 1280 triangles is faster shared.
+// Triangles few enough to test one after the other, the lanes together.
+// Measured on path tracing of a box around one such boundary, 512x512, the four
+// path kernels, one after the other / shared walks: 8 triangles 4.06 / 4.15 ms,
+// 12 4.23 / 4.49, 20 4.56 / 4.88, 32 4.87 / 4.94, 48 5.26 / 5.00, 80 6.01 / 5.34,
+// 1280 43.4 / 6.1.  The two cross near 35 triangles; the line lies below that.
 constexpr unsigned kFewTriangles = 16;
 struct AllHitsStack {
     int link[kAllHitsStack];

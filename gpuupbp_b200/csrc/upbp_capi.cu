@@ -960,9 +960,14 @@ int sort_queries(upbp_ctx* c, int q, unsigned n, const unsigned** order)
     unsigned** b = c->d_sort[q];
     cub::DoubleBuffer<unsigned> kb(b[0], b[1]), vb(b[2], b[3]);
     size_t tb = c->sort_temp_bytes;
-    // Few queries: the upper bits alone, a pass of about 9 us for every 8
-    // (preview 64x64: 7 instead of 12 passes); their cells already hold less
-    // than one query on average, so the finer bits order next to nothing.
+    // Few queries: the upper bits alone.  A radix pass of about 9 us sorts 8
+    // bits, and the finer cells it would order save less than that in walks shared
+    // by neighbours (a whole pass of the box at 6k, 36k and 92k segment queries:
+    // 2.16, 5.20, 17.7 ms with all bits, 2.09, 5.14, 17.4 without the lower 28,
+    // 2.08, 5.13, 17.7 without 36).  Many queries: the walks cost more (the media
+    // field at 834k and 1.48M: 18.5 and 36.7 ms with all bits, 18.8 and 37.7 without
+    // 28).  From 90k to 370k the two agree within the runs' spread, so the line
+    // lies there; the lower one, where 28 and 36 agree within 0.5%.
     const int drop = n <= 16384u ? (q == 0 ? 36 : 6) : n <= 131072u ? (q == 0 ? 28 : 6) : 0;
     if (q == 0) {
         cub::DoubleBuffer<unsigned long long> kb64((unsigned long long*)b[0], (unsigned long long*)b[1]);
