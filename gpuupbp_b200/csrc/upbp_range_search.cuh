@@ -23,10 +23,10 @@
 // reporting rule alone, so the accepted pairs are those of any other walk.
 //
 // Measured, BB1D search and evaluation, before -> now: media field at
-// 1280x720 24.2 -> 17.9 ms (search 12.3: 472M four-wide node tests instead of
-// 1393M two-wide ones), box 256x256 25.1 -> 11.4, dense beams 480x270 55.3 ->
-// 43.6, 64x64 preview 1.32 -> 0.13 ms.  What bounds it now: issue (55-70%) and
-// the L1 data pipe (60-75%) together; on the dense beams the L2, whose 126 MB
+// 1280x720 24.2 -> 16.0 ms (search 11.1: 456M four-wide node tests instead of
+// 1393M two-wide ones), box 256x256 25.1 -> 11.1, dense beams 480x270 55.3 ->
+// 42.3, 64x64 preview 1.32 -> 0.13 ms.  What bounds it now: issue (71%) and
+// the L1 data pipe (85%) together; on the dense beams the L2, whose 126 MB
 // the map and the query records share.
 #pragma once
 
