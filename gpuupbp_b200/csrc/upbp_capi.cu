@@ -2263,6 +2263,7 @@ extern "C" int upbp_debug_search(upbp_ctx* c, int kind, const float* queries, ui
                 cudaStreamSynchronize(c->st);
                 void* b[] = {q, counts, ids, words, seg, pt, work};
                 for (void* x : b) cudaFree(x);
+                (void)cudaGetLastError();  // an allocation that failed is reported by the call, not by the next one
                 c->P = keep;
             }
         } t(c);
